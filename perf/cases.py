@@ -143,7 +143,7 @@ def _light_maps(case, seed):
     """One map per light, its side and its scene's box count spread evenly
     over the case's range (sides 2^lo .. 2^hi, 10 .. 2000 boxes)."""
     g, sides = _rng(seed), case["hi"] - case["lo"] + 1
-    return [_map(1 << (case["lo"] + i % sides), int(10 * 200 ** (i * 7 % 16 / 15)), 0, g)
+    return [_map(1 << (case["lo"] + i * 5 % sides), int(10 * 200 ** (i * 7 % 16 / 15)), 0, g)
             for i in range(case["lights"])]
 
 
@@ -329,7 +329,7 @@ def work(case):
         return {"bytes": b * 1.036, "flops": 0}
     if k == "lights":
         sides = case["hi"] - case["lo"] + 1
-        b = sum(4 * (1 << (case["lo"] + i % sides)) ** 2 for i in range(case["lights"]))
+        b = sum(4 * (1 << (case["lo"] + i * 5 % sides)) ** 2 for i in range(case["lights"]))
         return {"bytes": b + case["points"] * 16.125, "flops": 0}
     if k == "grid":
         return {"bytes": 4 * (case["length"] * case["n"]) ** 2 + case["points"] * 12.125, "flops": 0}
