@@ -2001,10 +2001,13 @@ __global__ void __launch_bounds__(kThreads)
         bool same = false;
         if (first) {
             lead = (uint32_t)__ffs((int)__match_any_sync(act, (uint32_t)h)) - 1u;
+            // (`&=`: every lane of `act` takes part in every exchange, whatever
+            // the ones before it gave)
             same = lead != lane;
-            same = __shfl_sync(act, m, (int)lead) == m && __shfl_sync(act, j, (int)lead) == j && same;
+            same &= __shfl_sync(act, m, (int)lead) == m;
+            same &= __shfl_sync(act, j, (int)lead) == j;
 #pragma unroll
-            for (uint32_t r = 0; r < 8; ++r) same = __shfl_sync(act, u[r], (int)lead) == u[r] && same;
+            for (uint32_t r = 0; r < 8; ++r) same &= __shfl_sync(act, u[r], (int)lead) == u[r];
         }
         uint32_t s = 0;
         if (!same) s = insert_probe<false>(cur, child, i, m, j, k, u, h, table, cap_mask, err);
