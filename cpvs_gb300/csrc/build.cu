@@ -4207,6 +4207,8 @@ cpvs_status build_dags(Ctx& ctx, const std::vector<SourceSpec>& sources, const s
             // level table
             plan_bind_tables(P);
             CPVS_CUDA(cudaMemcpyAsync(P->lvt, P->lv, sizeof(P->lv), cudaMemcpyHostToDevice, st));
+            // the plan's next build, maybe on another stream, waits for the table too
+            CPVS_CUDA(cudaEventRecord(P->done, st));
         }
     }
     float tuning_ms = 0.f;
