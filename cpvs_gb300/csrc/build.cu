@@ -3209,7 +3209,7 @@ struct BuildPlan {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;  // recorded after the emission that last read the scratch
     // fork / join of the ranking passes' stream in the captured launch sequence
-    cudaEvent_t fork[CPVS_MAX_LEVELS] = {nullptr}, join = nullptr, start = nullptr, tables = nullptr, leaf_join = nullptr;
+    cudaEvent_t fork[CPVS_MAX_LEVELS] = {nullptr}, join = nullptr, start = nullptr, cleared = nullptr, tables = nullptr, leaf_join = nullptr;
     bool tables_tuned = false;
     // single-pass levels: the levels >= small_lo run in the single-block
     // kernels; look-back tickets and flags (zeroed by every build)
@@ -3234,7 +3234,7 @@ void plan_release(Ctx& ctx, BuildPlan* P) {
     P->exec = nullptr;
     for (cudaEvent_t& e : P->fork)
         if (e) cudaEventDestroy(e), e = nullptr;
-    for (cudaEvent_t* e : {&P->join, &P->start, &P->tables, &P->leaf_join})
+    for (cudaEvent_t* e : {&P->join, &P->start, &P->cleared, &P->tables, &P->leaf_join})
         if (*e) cudaEventDestroy(*e), *e = nullptr;
     if (P->arena) ctx.release(P->arena, P->arena_bytes, true, nullptr);
     if (P->colrec) ctx.release(P->colrec, P->colrec_cap * 2 * sizeof(uint4), true, nullptr);
@@ -3529,6 +3529,27 @@ cpvs_status plan_enqueue(BuildPlan* P, cudaStream_t st, cudaStream_t rank_st, cu
         }
         CPVS_CUDA(clear(cr, rank_st));
     }
+    // results, level counts, job bases, look-back tickets and flags (the
+    // last two adjacent in the arena): before the first pass of either branch
+    // that may report an error there
+    {
+        KernelTimer kt(tm, K_TABLE_CLEAR, st);
+        ClearRanges cr{};
+        cr.p[0] = P->res;
+        cr.n[0] = result_bytes(njobs);
+        cr.p[1] = reinterpret_cast<char*>(P->counts);
+        cr.n[1] = CPVS_MAX_LEVELS * 4;
+        cr.p[2] = reinterpret_cast<char*>(P->segbuf + 6 * segn);
+        cr.n[2] = segn * 4;
+        cr.p[3] = reinterpret_cast<char*>(P->tickets);
+        cr.n[3] = reinterpret_cast<const char*>(P->flags + P->flags_count) - reinterpret_cast<const char*>(P->tickets);
+        CPVS_CUDA(clear(cr, st));
+    }
+    if (forked) {
+        CPVS_CUDA(event(P->cleared));
+        CPVS_CUDA(cudaEventRecord(P->cleared, st));
+        CPVS_CUDA(cudaStreamWaitEvent(rank_st, P->cleared, 0));
+    }
     // the leaf classes of every column, beside the expansion (they need
     // only the maps, their level-3 bounds and the cleared tables)
     if (P->leafmasks) {
@@ -3554,21 +3575,6 @@ cpvs_status plan_enqueue(BuildPlan* P, cudaStream_t st, cudaStream_t rank_st, cu
                                 err));
     }
     if (forked) CPVS_CUDA(cudaEventRecord(P->tables, rank_st));
-    // results, level counts, job bases, look-back tickets and flags (the
-    // last two adjacent in the arena)
-    {
-        KernelTimer kt(tm, K_TABLE_CLEAR, st);
-        ClearRanges cr{};
-        cr.p[0] = P->res;
-        cr.n[0] = result_bytes(njobs);
-        cr.p[1] = reinterpret_cast<char*>(P->counts);
-        cr.n[1] = CPVS_MAX_LEVELS * 4;
-        cr.p[2] = reinterpret_cast<char*>(P->segbuf + 6 * segn);
-        cr.n[2] = segn * 4;
-        cr.p[3] = reinterpret_cast<char*>(P->tickets);
-        cr.n[3] = reinterpret_cast<const char*>(P->flags + P->flags_count) - reinterpret_cast<const char*>(P->tickets);
-        CPVS_CUDA(clear(cr, st));
-    }
     // top-down: the small top levels as one cluster (which also places the
     // roots), then one pass per level
     const int Ls = P->small_lo;

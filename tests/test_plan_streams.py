@@ -1,6 +1,7 @@
-"""A plan's builds on several streams: what one build leaves for the next is
-ordered by the plan's event alone, so everything that it leaves comes before
-the event's last record."""
+"""The order of a build's work over streams.  What one build of a plan leaves
+for the next is ordered by the plan's event alone, so everything that it leaves
+comes before the event's last record.  Within a build, the word that errors are
+reported in is cleared before any branch may report one."""
 import os
 import re
 
@@ -23,6 +24,34 @@ def body(name):
 def test_the_level_table_is_copied_before_the_plans_event():
     b = body("build_dags")
     assert b.rindex("cudaMemcpyAsync(P->lvt") < b.rindex("cudaEventRecord(P->done")
+
+
+def test_the_error_word_is_cleared_before_the_leaf_branch():
+    b = body("plan_enqueue")
+    clear, leaves = b.index("= P->res;"), b.index("k_leaf_columns<true>")
+    assert clear < b.index("cudaStreamWaitEvent(rank_st, P->cleared") < leaves
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("timing", [False, True])
+def test_a_full_class_table_is_reported(cp, oracle, timing):
+    """The same 8x8 texels in every column, whose few leaf classes size the
+    table, then other ones in each column of a half and again in the other half:
+    more classes than it holds, while no level outgrows the plan and the inner
+    levels' tables suffice."""
+    n = 256
+    rng = np.random.default_rng(3)
+    tile = rng.uniform(0.3, 0.42, (8, 8)).astype(np.float32)
+    alike = np.tile(tile, (n // 8, n // 8))
+    # each column's texels in another order: the same bounds, so the same nodes
+    half = np.block([[rng.permutation(tile.ravel()).reshape(8, 8) for _ in range(n // 16)] for _ in range(n // 8)])
+    other = np.concatenate([half, half], 1)
+    ctx = cp.Context(0)
+    ctx.enable_timing(timing)
+    for k, d in enumerate((alike, np.ascontiguousarray(other))):
+        sh = cp.CompressedShadow.from_depth(d, ctx=ctx)
+        assert np.array_equal(sh.get_dag(), oracle.build(d).dag)
+        assert ctx.last_build()["replans"] == k
 
 
 @pytest.mark.gpu
