@@ -4361,6 +4361,7 @@ extern "C" CPVS_API cpvs_status cpvs_shadow_build_noalloc(const float* depth, ui
     uint64_t* job_off = A.take<uint64_t>(2);
     uint32_t* root_dev = A.take<uint32_t>(1);
     JobDev* job_dev = A.take<JobDev>(1);
+    float* own = aligned16(depth) ? nullptr : A.take<float>((size_t)n * n);
     if (A.used > A.size)
         return fail(CPVS_ERR_INVALID_ARG, "noalloc: this map needs " + std::to_string(A.used) +
                                               " scratch bytes, above the fixed " +
@@ -4373,6 +4374,10 @@ extern "C" CPVS_API cpvs_status cpvs_shadow_build_noalloc(const float* depth, ui
     CPVS_CUDA(cudaMemsetAsync(counts, 0, CPVS_MAX_LEVELS * sizeof(uint32_t), st));
     CPVS_CUDA(cudaMemsetAsync(level_u, 0, 2 * CPVS_MAX_LEVELS * sizeof(uint32_t), st));
     CPVS_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
+    if (own) {
+        CPVS_CUDA(cudaMemcpyAsync(own, depth, (size_t)n * n * sizeof(float), cudaMemcpyDeviceToDevice, st));
+        depth = own;
+    }
     r = launch_pyramid(depth, n, pyr, st);
     if (r != CPVS_OK) return r;
     const JobDev jd{pyr, depth, n, (uint32_t)nl, z_tile_index, z_tile_num};

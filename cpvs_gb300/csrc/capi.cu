@@ -499,7 +499,7 @@ cpvs_status hierarchy_create(cpvs_ctx* ctx, const float* depth, uint32_t n, uint
     auto* h = new cpvs_hierarchy(ctx);
     h->n = n;
     h->first_level = first_level;
-    const bool borrow = (flags & CPVS_IO_DEVICE) && (flags & CPVS_FLAG_BORROW_INPUT);
+    const bool borrow = (flags & CPVS_IO_DEVICE) && (flags & CPVS_FLAG_BORROW_INPUT) && cpvs::aligned16(depth);
     if (borrow) {
         h->depth = const_cast<float*>(depth);
         h->owns_depth = false;
@@ -512,34 +512,31 @@ cpvs_status hierarchy_create(cpvs_ctx* ctx, const float* depth, uint32_t n, uint
         if (r == CPVS_OK) h->bytes += lbytes;
     }
     // a host map the GPU reads in place is copied by the pyramid kernel as
-    // it reduces it (one pass over the host link); any other host map is
-    // uploaded first
-    const float* in_place = (!(flags & CPVS_IO_DEVICE) && r == CPVS_OK)
-                                ? static_cast<const float*>(cpvs::host_accessible(c, depth))
-                                : nullptr;
+    // it reduces it (one pass over the host link); any other host map, and one
+    // off a 16-byte boundary, is uploaded first
+    const float* reached = (!(flags & CPVS_IO_DEVICE) && r == CPVS_OK)
+                               ? static_cast<const float*>(cpvs::host_accessible(c, depth))
+                               : nullptr;
+    const float* in_place = cpvs::aligned16(reached) ? reached : nullptr;
     if (r == CPVS_OK && !borrow && !in_place) {
         cudaError_t e = cudaMemcpyAsync(h->depth, depth, dbytes,
                                         (flags & CPVS_IO_DEVICE) ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st);
         if (e != cudaSuccess) r = cpvs::cuda_fail(e, "hierarchy upload");
     }
-    if (r == CPVS_OK) {
-        if (in_place) {
-            r = cpvs::launch_pyramid(in_place, n, h->levels, st, &c.timing, h->depth, first_level,
-                                     cpvs::pyramid_nan_flag(h->levels, n));
-            // the caller may reuse its buffer on return: wait for the read
-            // (or hand the wait to the caller)
-            if (r == CPVS_OK && host_read) {
-                cudaError_t e = cudaEventCreateWithFlags(host_read, cudaEventDisableTiming);
-                if (e == cudaSuccess) e = cudaEventRecord(*host_read, st);
-                if (e != cudaSuccess) r = cpvs::cuda_fail(e, "hierarchy read of the host map");
-            }
-            if (r != CPVS_OK || !host_read) {
-                const cudaError_t e = cudaStreamSynchronize(st);
-                if (e != cudaSuccess && r == CPVS_OK) r = cpvs::cuda_fail(e, "hierarchy read of the host map");
-            }
-        } else {
-            r = cpvs::launch_pyramid(h->depth, n, h->levels, st, &c.timing, nullptr, first_level,
-                                     cpvs::pyramid_nan_flag(h->levels, n));
+    if (r == CPVS_OK)
+        r = cpvs::launch_pyramid(in_place ? in_place : h->depth, n, h->levels, st, &c.timing,
+                                 in_place ? h->depth : nullptr, first_level, cpvs::pyramid_nan_flag(h->levels, n));
+    if (reached) {
+        // the caller may reuse its buffer on return: wait for the read (or
+        // hand the wait to the caller)
+        if (r == CPVS_OK && host_read) {
+            cudaError_t e = cudaEventCreateWithFlags(host_read, cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventRecord(*host_read, st);
+            if (e != cudaSuccess) r = cpvs::cuda_fail(e, "hierarchy read of the host map");
+        }
+        if (r != CPVS_OK || !host_read) {
+            const cudaError_t e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess && r == CPVS_OK) r = cpvs::cuda_fail(e, "hierarchy read of the host map");
         }
     }
     h->touch(st);
@@ -587,7 +584,7 @@ cpvs_status cpvs_hierarchy_create_batch(cpvs_ctx* ctx, const float* const* depth
         h->first_level = 1;
         hs.push_back(h);
         const uint64_t dbytes = (uint64_t)n * n * 4, lbytes = cpvs::pyramid_bytes(n);
-        if (borrow) {
+        if (borrow && cpvs::aligned16(depths[i])) {
             h->depth = const_cast<float*>(depths[i]);
             h->owns_depth = false;
         } else {

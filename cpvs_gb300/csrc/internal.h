@@ -57,6 +57,9 @@ inline uint64_t pyramid_bytes(uint32_t n) { return pyramid_texels(n) * 8 + 32; }
 inline uint32_t* pyramid_nan_flag(float2* levels, uint32_t n) {
     return reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(levels) + pyramid_texels(n) * 8 + 16);
 }
+// The build's kernels read a map in 16-byte loads; a map that begins elsewhere
+// (a view into a larger buffer) is copied first.
+inline bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 inline int log2_u32(uint32_t n) {
     int l = 0;
     while ((1u << l) < n) ++l;

@@ -115,8 +115,6 @@ __global__ void __launch_bounds__(kShadeThreads) k_shade(ShadeArgs a) {
     }
 }
 
-bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
-
 }  // namespace
 
 cpvs_status launch_shade(uint64_t n, const float* normals, uint32_t normal_floats, const float* albedo,

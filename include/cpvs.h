@@ -71,7 +71,9 @@ typedef enum cpvs_visibility {
 #define CPVS_FLAG_BORROW_INPUT 0x200u  /* with CPVS_IO_DEVICE: a hierarchy reads the
                                           caller's depth map in place instead of
                                           copying it; the caller keeps it alive and
-                                          unchanged until the hierarchy is destroyed */
+                                          unchanged until the hierarchy is destroyed.
+                                          A map off a 16-byte boundary (a view into
+                                          a larger buffer) is copied all the same */
 
 typedef struct cpvs_ctx cpvs_ctx;
 typedef struct cpvs_hierarchy cpvs_hierarchy;
