@@ -37,15 +37,25 @@ struct DeviceObject {
         }
         if (use_->event) cudaEventRecord(use_->event, st);
     }
-    // One record for all of `objects` (of one context).
+    // One record for all of `objects` of the first one's context; those of
+    // another one (a batch may build from several contexts' hierarchies) have
+    // their own, from that context's pool and under its mutex.
     template <class T>
     static void touch_all(T* const* objects, size_t count, cudaStream_t st) {
         if (!count) return;
         cpvs::Ctx* c = objects[0]->c_;
+        uint32_t mine = 0;
+        for (size_t i = 0; i < count; ++i) {
+            if (objects[i]->c_ == c)
+                ++mine;
+            else
+                objects[i]->touch(st);
+        }
         std::lock_guard<std::mutex> lock(c->event_mutex);
-        auto* u = new UseEvent{c->take_event(), (uint32_t)count};
+        auto* u = new UseEvent{c->take_event(), mine};
         if (u->event) cudaEventRecord(u->event, st);
         for (size_t i = 0; i < count; ++i) {
+            if (objects[i]->c_ != c) continue;
             objects[i]->drop();
             objects[i]->use_ = u;
         }
