@@ -3250,6 +3250,15 @@ void plan_release(Ctx& ctx, BuildPlan* P) {
     P->staged.clear();
 }
 
+// Releases a plan of the context's cache and takes it out of there.
+void plan_drop(Ctx& ctx, BuildPlan* P) {
+    plan_release(ctx, P);
+    if (P->done) cudaEventDestroy(P->done);
+    auto& plans = ctx.plans->plans;
+    plans.erase(std::find(plans.begin(), plans.end(), P));
+    delete P;
+}
+
 // Per-level table regions (consecutive, tcap[L] slots each) and the split
 // between the multi-block levels and the topmost ones that run in the
 // cluster kernels (a level is small when it and every level above it hold
@@ -3286,6 +3295,8 @@ uint64_t plan_table_slots(const BuildPlan* P) {
 // Capacities -> scratch layout, pinned staging, level table.
 cpvs_status plan_allocate(Ctx& ctx, BuildPlan* P, cudaStream_t st) {
     const uint32_t njobs = P->njobs;
+    for (int L = 0; L < CPVS_MAX_LEVELS; ++L)
+        if (P->cap[L] >= (1ull << 31)) return fail(CPVS_ERR_BUDGET, "build: a level exceeds 2^31 nodes");
     const size_t segn = (size_t)njobs * CPVS_MAX_LEVELS;
     size_t bytes = 0;
     auto add = [&](size_t count, size_t elem) { bytes += align256(count * elem); };
@@ -3902,11 +3913,6 @@ cpvs_status plan_create(Ctx& ctx, const std::vector<JobSpec>& jobs, const std::v
     }
     P->inj_off[CPVS_MAX_LEVELS] = o;
     plan_set_capacities(P, bounds, true);
-    for (int L = 0; L < CPVS_MAX_LEVELS; ++L)
-        if (P->cap[L] >= (1ull << 31)) {
-            delete P;
-            return fail(CPVS_ERR_BUDGET, "build: a level exceeds 2^31 nodes");
-        }
     cpvs_status r = plan_allocate(ctx, P, st);
     if (r != CPVS_OK) {
         plan_release(ctx, P);
@@ -4000,12 +4006,7 @@ cpvs_status build_dags(Ctx& ctx, const std::vector<SourceSpec>& sources, const s
         if (r == CPVS_OK) P->pow2 = pow2;
         if (r != CPVS_OK) return r;
         // keep a few shapes; drop the oldest
-        if (ctx.plans->plans.size() >= 8) {
-            plan_release(ctx, ctx.plans->plans.front());
-            if (ctx.plans->plans.front()->done) cudaEventDestroy(ctx.plans->plans.front()->done);
-            delete ctx.plans->plans.front();
-            ctx.plans->plans.erase(ctx.plans->plans.begin());
-        }
+        if (ctx.plans->plans.size() >= 8) plan_drop(ctx, ctx.plans->plans.front());
         ctx.plans->plans.push_back(P);
     }
 
@@ -4147,7 +4148,12 @@ cpvs_status build_dags(Ctx& ctx, const std::vector<SourceSpec>& sources, const s
         plan_release(ctx, P);
         plan_set_capacities(P, bounds, true);
         cpvs_status r = plan_allocate(ctx, P, st);
-        if (r != CPVS_OK) return r;
+        if (r != CPVS_OK) {
+            // no room to grow: without its scratch the plan is of no use to
+            // the next build of this shape, which makes another
+            plan_drop(ctx, P);
+            return r;
+        }
     }
 
     const size_t segn = (size_t)njobs * CPVS_MAX_LEVELS;
