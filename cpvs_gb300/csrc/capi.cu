@@ -26,70 +26,6 @@ cpvs_status cuda_fail(cudaError_t e, const char* what) {
     return fail(s, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// A pool that holds on to `keep` bytes, freed blocks included, before it returns
-// any to the CUDA driver.
-static cudaError_t create_pool(int device, cudaMemPool_t* pool, uint64_t keep) {
-    cudaMemPoolProps props{};
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = device;
-    const cudaError_t e = cudaMemPoolCreate(pool, &props);
-    if (e == cudaSuccess) cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    return e;
-}
-
-cpvs_status Ctx::alloc(void** p, uint64_t bytes, bool persistent, cudaStream_t st, cudaMemPool_t from) {
-    *p = nullptr;
-    if (budget && in_use + scratch + bytes > budget)
-        return fail(CPVS_ERR_BUDGET, "allocation of " + std::to_string(bytes) + " bytes exceeds the context budget");
-    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, from ? from : pool, st);
-    if (e == cudaErrorMemoryAllocation && index_pool && cudaMemPoolTrimTo(index_pool, 0) == cudaSuccess) {
-        cudaGetLastError();
-        e = cudaMallocFromPoolAsync(p, bytes, from ? from : pool, st);
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocFromPoolAsync");
-    if (persistent)
-        in_use += bytes;
-    else
-        scratch += bytes;
-    return CPVS_OK;
-}
-
-cudaEvent_t Ctx::take_event() {
-    if (!event_pool.empty()) {
-        const cudaEvent_t e = event_pool.back();
-        event_pool.pop_back();
-        return e;
-    }
-    cudaEvent_t e = nullptr;
-    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return e;
-}
-
-void Ctx::give_event(cudaEvent_t e) {
-    if (!e) return;
-    if (event_pool.size() < kEventPool)
-        event_pool.push_back(e);
-    else
-        cudaEventDestroy(e);
-}
-
-void Ctx::release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cudaEvent_t last_use) {
-    if (persistent) {
-        if (p) {
-            if (last_use) cudaStreamWaitEvent(free_stream, last_use, 0);
-            cudaFreeAsync(p, free_stream);
-        }
-        in_use -= std::min(in_use, bytes);
-    } else {
-        if (p) cudaFreeAsync(p, st);
-        scratch -= std::min(scratch, bytes);
-    }
-}
-
 }  // namespace cpvs
 
 using cpvs::fail;
@@ -252,17 +188,6 @@ cpvs_status build_into_shadows(cpvs_ctx* ctx, const std::vector<cpvs::SourceSpec
 // a pool of their own, as the containers' have: the next one takes the place of
 // one that was freed, where in the context's pool a build's blocks lay in its
 // way and the pool grew (70 us and more).
-constexpr uint64_t kIndexKeep = 1ull << 30;  // 16 of the largest
-cudaMemPool_t indices_from(cpvs::Ctx& c, cudaStream_t st) {
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone ||
-        (!c.index_pool && cpvs::create_pool(c.device, &c.index_pool, kIndexKeep) != cudaSuccess)) {
-        cudaGetLastError();
-        return nullptr;  // (no pool is made during a capture)
-    }
-    return c.index_pool;
-}
-
 constexpr uint32_t kTopFactor = 8;
 void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor = kTopFactor,
                  uint64_t points = 0) {
@@ -272,7 +197,7 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
         cpvs_shadow* s = const_cast<cpvs_shadow*>(shadows[i]);
         if (s->top || s->top_bytes == ~0ull) continue;
         cpvs::Ctx& c = s->ctx->c;
-        if (points && !indices_from(c, st)) points = 0;
+        if (points && !c.index_source(st)) points = 0;
         const int least = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, 0);
         int depth = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, c.budget ? 0 : points / 2);
         while (depth > 0 && c.alloc((void**)&s->top, uint64_t(4) << (3 * depth), true, st,
@@ -408,7 +333,7 @@ void cpvs_ctx_destroy(cpvs_ctx* ctx) {
 
 cpvs_status cpvs_ctx_set_budget(cpvs_ctx* ctx, uint64_t bytes) {
     if (!ctx) return fail(CPVS_ERR_INVALID_ARG, "null ctx");
-    ctx->c.budget = bytes;
+    ctx->c.set_budget(bytes);
     return CPVS_OK;
 }
 
@@ -1169,7 +1094,7 @@ static void ensure_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     const int depth = cpvs::grid_top_depth(g->length, g->dag_levels, g->leafmasks, g->words);
     const uint64_t bytes = uint64_t(4) << (3 * (cpvs::log2_u32(g->length) + depth));
     if (depth <= 0 ||
-        g->ctx->c.alloc((void**)&g->gtop, bytes, true, st, indices_from(g->ctx->c, st)) != CPVS_OK ||
+        g->ctx->c.alloc((void**)&g->gtop, bytes, true, st, g->ctx->c.index_source(st)) != CPVS_OK ||
         cpvs::launch_grid_top_index(g->dag, g->words, g->cell_words, g->length, g->dag_levels, depth, g->gtop, st) !=
             CPVS_OK) {
         if (g->gtop) g->ctx->c.release(g->gtop, bytes, true, st);

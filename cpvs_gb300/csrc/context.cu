@@ -1,0 +1,94 @@
+// A context's device memory: its pools, the budget's accounting, and the events
+// of its objects' last uses.
+#include <algorithm>
+
+#include "internal.h"
+
+namespace cpvs {
+
+cudaError_t create_pool(int device, cudaMemPool_t* pool, uint64_t keep) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    const cudaError_t e = cudaMemPoolCreate(pool, &props);
+    if (e == cudaSuccess) cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    return e;
+}
+
+cpvs_status Ctx::alloc(void** p, uint64_t bytes, bool persistent, cudaStream_t st, cudaMemPool_t from) {
+    *p = nullptr;
+    if (budget && in_use + scratch + bytes > budget)
+        return fail(CPVS_ERR_BUDGET, "allocation of " + std::to_string(bytes) + " bytes exceeds the context budget");
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, from ? from : pool, st);
+    if (e == cudaErrorMemoryAllocation && index_pool && cudaMemPoolTrimTo(index_pool, 0) == cudaSuccess) {
+        cudaGetLastError();
+        e = cudaMallocFromPoolAsync(p, bytes, from ? from : pool, st);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocFromPoolAsync");
+    if (persistent)
+        in_use += bytes;
+    else
+        scratch += bytes;
+    return CPVS_OK;
+}
+
+cudaEvent_t Ctx::take_event() {
+    if (!event_pool.empty()) {
+        const cudaEvent_t e = event_pool.back();
+        event_pool.pop_back();
+        return e;
+    }
+    cudaEvent_t e = nullptr;
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return e;
+}
+
+void Ctx::give_event(cudaEvent_t e) {
+    if (!e) return;
+    if (event_pool.size() < kEventPool)
+        event_pool.push_back(e);
+    else
+        cudaEventDestroy(e);
+}
+
+void Ctx::release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cudaEvent_t last_use) {
+    if (persistent) {
+        if (p) {
+            if (last_use) cudaStreamWaitEvent(free_stream, last_use, 0);
+            cudaFreeAsync(p, free_stream);
+        }
+        in_use -= std::min(in_use, bytes);
+    } else {
+        if (p) cudaFreeAsync(p, st);
+        scratch -= std::min(scratch, bytes);
+    }
+}
+
+// 16 of the largest indices.
+constexpr uint64_t kIndexKeep = 1ull << 30;
+
+cudaMemPool_t Ctx::index_source(cudaStream_t st) {
+    if (budget) return nullptr;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone ||
+        (!index_pool && create_pool(device, &index_pool, kIndexKeep) != cudaSuccess)) {
+        cudaGetLastError();
+        return nullptr;  // (no pool is made during a capture)
+    }
+    return index_pool;
+}
+
+void Ctx::set_budget(uint64_t bytes) {
+    budget = bytes;
+    if (!index_pool) return;
+    uint64_t keep = budget ? 0 : kIndexKeep;
+    cudaMemPoolSetAttribute(index_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (budget) cudaMemPoolTrimTo(index_pool, 0);
+    cudaGetLastError();
+}
+
+}  // namespace cpvs

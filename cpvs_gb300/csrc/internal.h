@@ -272,6 +272,10 @@ struct KernelTimer {
 };
 
 // ----------------------------------------------------------------- ctx
+// A pool that holds on to `keep` bytes, freed blocks included, before it returns
+// any to the CUDA driver.
+cudaError_t create_pool(int device, cudaMemPool_t* pool, uint64_t keep);
+
 struct Ctx {
     Timing timing;
     int device = 0;
@@ -311,6 +315,12 @@ struct Ctx {
     std::vector<cudaEvent_t> event_pool;
     cudaEvent_t take_event();
     void give_event(cudaEvent_t e);
+    // The pool that a large top grid is taken from; null: the context's own.
+    // With a budget that is always so: a second pool would hold its freed
+    // blocks beside the budget's.
+    cudaMemPool_t index_source(cudaStream_t st);
+    // The limit, 0 for none.  Under a limit the second pool holds no freed blocks.
+    void set_budget(uint64_t bytes);
     // Allocation on stream `st`, with budget accounting.
     cpvs_status alloc(void** p, uint64_t bytes, bool persistent, cudaStream_t st, cudaMemPool_t from = nullptr);
     // Scratch: freed in the order of `st`.  Persistent: freed once

@@ -1,0 +1,124 @@
+// A context's memory over its two pools (csrc/context.cu), with a model of the
+// CUDA pools in place of the driver's: a device of `capacity` bytes, pools that
+// reserve what they hand out and keep what is freed up to their threshold.
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <string>
+#include <vector>
+
+namespace model {
+constexpr uint64_t MiB = 1ull << 20;
+uint64_t capacity = 1024 * MiB;
+struct Pool {
+    uint64_t reserved = 0, used = 0, keep = 0;
+};
+std::vector<Pool*> pools;
+std::map<void*, std::pair<Pool*, uint64_t>> blocks;
+bool capturing = false;
+char place[1 << 12];
+size_t next = 0;
+
+uint64_t reserved() {
+    uint64_t r = 0;
+    for (const Pool* p : pools) r += p->reserved;
+    return r;
+}
+cudaError_t create(cudaMemPool_t* out, const cudaMemPoolProps*) {
+    pools.push_back(new Pool);
+    *out = reinterpret_cast<cudaMemPool_t>(pools.back());
+    return cudaSuccess;
+}
+cudaError_t attribute(cudaMemPool_t p, cudaMemPoolAttr, void* v) {
+    reinterpret_cast<Pool*>(p)->keep = *static_cast<uint64_t*>(v);
+    return cudaSuccess;
+}
+cudaError_t trim(cudaMemPool_t p, size_t) {
+    Pool* q = reinterpret_cast<Pool*>(p);
+    q->reserved = q->used;
+    return cudaSuccess;
+}
+cudaError_t allocate(void** out, size_t bytes, cudaMemPool_t p, cudaStream_t) {
+    Pool* q = reinterpret_cast<Pool*>(p);
+    const uint64_t more = q->used + bytes > q->reserved ? q->used + bytes - q->reserved : 0;
+    if (reserved() + more > capacity) return cudaErrorMemoryAllocation;
+    q->reserved += more;
+    q->used += bytes;
+    *out = place + next++;
+    blocks[*out] = {q, bytes};
+    return cudaSuccess;
+}
+cudaError_t release(void* p, cudaStream_t) {
+    auto b = blocks[p];
+    blocks.erase(p);
+    b.first->used -= b.second;
+    if (b.first->reserved > b.first->keep) b.first->reserved = b.first->used > b.first->keep ? b.first->used : b.first->keep;
+    return cudaSuccess;
+}
+cudaError_t is_capturing(cudaStream_t, cudaStreamCaptureStatus* s) {
+    *s = capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    return cudaSuccess;
+}
+cudaError_t ok() { return cudaSuccess; }
+}  // namespace model
+
+#define cudaMemPoolCreate model::create
+#define cudaMemPoolSetAttribute model::attribute
+#define cudaMemPoolTrimTo model::trim
+#define cudaMallocFromPoolAsync model::allocate
+#define cudaFreeAsync model::release
+#define cudaStreamIsCapturing model::is_capturing
+#define cudaGetLastError model::ok
+#include "../../cpvs_gb300/csrc/context.cu"
+
+namespace cpvs {
+cpvs_status fail(cpvs_status s, const std::string&) { return s; }
+cpvs_status cuda_fail(cudaError_t e, const char*) {
+    return e == cudaErrorMemoryAllocation ? CPVS_ERR_OOM : CPVS_ERR_DEVICE;
+}
+}  // namespace cpvs
+
+using model::MiB;
+
+static void check(bool ok, const char* what) {
+    if (ok) return;
+    std::printf("failed: %s\n", what);
+    std::exit(1);
+}
+
+static void begin(cpvs::Ctx& c) { cpvs::create_pool(0, &c.pool, ~0ull); }
+
+// Under a budget nothing is held outside the budget's own pool.
+static void budget() {
+    cpvs::Ctx c;
+    begin(c);
+    void* p = nullptr;
+    check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(nullptr)) == CPVS_OK, "an index without a budget");
+    c.release(p, 64 * MiB, true, nullptr);
+    void* held = nullptr;
+    check(c.alloc(&held, 64 * MiB, true, nullptr, c.index_source(nullptr)) == CPVS_OK, "an index without a budget");
+    c.set_budget(200 * MiB);
+    check(c.index_source(nullptr) == nullptr, "an index under a budget comes from the context's pool");
+    check(model::reserved() == 64 * MiB, "freed blocks of the second pool go back with a budget");
+    c.release(held, 64 * MiB, true, nullptr);
+    check(model::reserved() == 0, "blocks of the second pool freed under a budget go back");
+    for (int k = 0; k < 4; ++k) {
+        check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(nullptr)) == CPVS_OK, "an index under a budget");
+        c.release(p, 64 * MiB, true, nullptr);
+        check(c.alloc(&p, 200 * MiB, true, nullptr) == CPVS_OK, "the whole budget");
+        c.release(p, 200 * MiB, true, nullptr);
+    }
+    check(model::reserved() <= 200 * MiB, "the device memory held stays within the budget");
+}
+
+int main(int argc, char** argv) {
+    const std::string what = argc > 1 ? argv[1] : "";
+    if (what == "budget") budget();
+    else return 2;
+    std::printf("ok\n");
+    return 0;
+}
