@@ -21,7 +21,11 @@ cpvs_status Ctx::alloc(void** p, uint64_t bytes, bool persistent, cudaStream_t s
     if (budget && in_use + scratch + bytes > budget)
         return fail(CPVS_ERR_BUDGET, "allocation of " + std::to_string(bytes) + " bytes exceeds the context budget");
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, from ? from : pool, st);
-    if (e == cudaErrorMemoryAllocation && index_pool && cudaMemPoolTrimTo(index_pool, 0) == cudaSuccess) {
+    if (e == cudaErrorMemoryAllocation && index_pool) {
+        // the freed blocks that one pool holds are no use to the other: back
+        // to the driver with both
+        cudaMemPoolTrimTo(index_pool, 0);
+        cudaMemPoolTrimTo(pool, 0);
         cudaGetLastError();
         e = cudaMallocFromPoolAsync(p, bytes, from ? from : pool, st);
     }

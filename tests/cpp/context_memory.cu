@@ -115,9 +115,26 @@ static void budget() {
     check(model::reserved() <= 200 * MiB, "the device memory held stays within the budget");
 }
 
+// What is free in one pool is there for the other where the device has no more.
+static void full() {
+    cpvs::Ctx c;
+    begin(c);
+    void *p = nullptr, *q = nullptr;
+    cudaMemPool_t second = c.index_source(nullptr);
+    check(second != nullptr, "a second pool");
+    check(c.alloc(&p, 1000 * MiB, false, nullptr) == CPVS_OK, "a large scratch");
+    c.release(p, 1000 * MiB, false, nullptr);
+    check(c.alloc(&p, 64 * MiB, true, nullptr, second) == CPVS_OK, "an index after it");
+    c.release(p, 64 * MiB, true, nullptr);
+    check(c.alloc(&p, 1000 * MiB, false, nullptr) == CPVS_OK, "the scratch again");
+    check(c.alloc(&q, 64 * MiB, true, nullptr, second) == CPVS_ERR_OOM, "no room for both");
+    c.release(p, 1000 * MiB, false, nullptr);
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "budget") budget();
+    else if (what == "full") full();
     else return 2;
     std::printf("ok\n");
     return 0;
