@@ -184,10 +184,7 @@ cpvs_status build_into_shadows(cpvs_ctx* ctx, const std::vector<cpvs::SourceSpec
 // later ones.  2^26 points, an 8192^2 map (first / later): 495 -> 441 / 466 ->
 // 393 us with 8 levels for 7; 2^25, a 2048^2 map of 45 objects: 231 -> 189 / 215
 // -> 156; 1.3 * 2^22 of them: 55 -> 49 / 45 -> 38; a cell per point gained nothing
-// more at 1.3 * 2^18 and lost 3% of the first lookup at 2^24.  These grids have
-// a pool of their own, as the containers' have: the next one takes the place of
-// one that was freed, where in the context's pool a build's blocks lay in its
-// way and the pool grew (70 us and more).
+// more at 1.3 * 2^18 and lost 3% of the first lookup at 2^24.
 constexpr uint32_t kTopFactor = 8;
 void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor = kTopFactor,
                  uint64_t points = 0) {
@@ -197,11 +194,12 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
         cpvs_shadow* s = const_cast<cpvs_shadow*>(shadows[i]);
         if (s->top || s->top_bytes == ~0ull) continue;
         cpvs::Ctx& c = s->ctx->c;
-        if (points && !c.index_source(st)) points = 0;
+        if (points && !c.index_beyond_rule(st)) points = 0;
         const int least = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, 0);
-        int depth = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, c.budget ? 0 : points / 2);
-        while (depth > 0 && c.alloc((void**)&s->top, uint64_t(4) << (3 * depth), true, st,
-                                    depth > least ? c.index_pool : nullptr) != CPVS_OK) {
+        int depth = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, points / 2);
+        auto bytes = [&] { return uint64_t(4) << (3 * depth); };
+        while (depth > 0 && c.alloc((void**)&s->top, bytes(), true, st,
+                                    depth > least ? c.index_source(bytes(), st) : nullptr) != CPVS_OK) {
             s->top = nullptr;
             cudaGetLastError();
             depth = depth > least ? least : 0;
@@ -210,7 +208,7 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
             s->top_bytes = ~0ull;  // look up without it
             continue;
         }
-        s->top_bytes = uint64_t(4) << (3 * depth);
+        s->top_bytes = bytes();
         s->top_depth = depth;
         grids.push_back(cpvs::TopGrid{s->dag, s->words, depth, s->top});
         owners.push_back(s);
@@ -1094,7 +1092,7 @@ static void ensure_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     const int depth = cpvs::grid_top_depth(g->length, g->dag_levels, g->leafmasks, g->words);
     const uint64_t bytes = uint64_t(4) << (3 * (cpvs::log2_u32(g->length) + depth));
     if (depth <= 0 ||
-        g->ctx->c.alloc((void**)&g->gtop, bytes, true, st, g->ctx->c.index_source(st)) != CPVS_OK ||
+        g->ctx->c.alloc((void**)&g->gtop, bytes, true, st, g->ctx->c.index_source(bytes, st)) != CPVS_OK ||
         cpvs::launch_grid_top_index(g->dag, g->words, g->cell_words, g->length, g->dag_levels, depth, g->gtop, st) !=
             CPVS_OK) {
         if (g->gtop) g->ctx->c.release(g->gtop, bytes, true, st);

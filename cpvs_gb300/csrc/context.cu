@@ -72,16 +72,24 @@ void Ctx::release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cud
     }
 }
 
-// 16 of the largest indices.
-constexpr uint64_t kIndexKeep = 1ull << 30;
+constexpr uint64_t kIndexOwn = 16ull << 20;
+constexpr uint64_t kIndexKeep = 1ull << 30;  // 16 of the largest
 
-cudaMemPool_t Ctx::index_source(cudaStream_t st) {
-    if (budget) return nullptr;
+bool Ctx::index_beyond_rule(cudaStream_t st) const {
+    if (budget) return false;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone ||
-        (!index_pool && create_pool(device, &index_pool, kIndexKeep) != cudaSuccess)) {
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
         cudaGetLastError();
-        return nullptr;  // (no pool is made during a capture)
+        return false;
+    }
+    return capturing == cudaStreamCaptureStatusNone;
+}
+
+cudaMemPool_t Ctx::index_source(uint64_t bytes, cudaStream_t st) {
+    if (bytes < kIndexOwn || !index_beyond_rule(st)) return nullptr;
+    if (!index_pool && create_pool(device, &index_pool, kIndexKeep) != cudaSuccess) {
+        cudaGetLastError();
+        index_pool = nullptr;
     }
     return index_pool;
 }

@@ -315,10 +315,18 @@ struct Ctx {
     std::vector<cudaEvent_t> event_pool;
     cudaEvent_t take_event();
     void give_event(cudaEvent_t e);
-    // The pool that a large top grid is taken from; null: the context's own.
-    // With a budget that is always so: a second pool would hold its freed
-    // blocks beside the budget's.
-    cudaMemPool_t index_source(cudaStream_t st);
+    // The pool that a top grid of `bytes` is taken from; null: the context's
+    // own.  The largest have a pool of their own, made for the first of them:
+    // the next one takes the place of one that was freed, where in the context's
+    // pool a build's blocks lay in its way and the pool grew.  Not the smaller
+    // ones, which find a place there: the second pool's making and its first
+    // memory cost a context's first lookup 150 to 250 us (first frame of a
+    // 1024^2 map 820 -> 1065 us, filtered 2048^2 628 -> 808).  Under a budget
+    // none: the pool would hold its freed blocks beside the budget's.
+    cudaMemPool_t index_source(uint64_t bytes, cudaStream_t st);
+    // Whether a top grid may be larger than the DAG's size allows (no budget, no
+    // capture on `st`).
+    bool index_beyond_rule(cudaStream_t st) const;
     // The limit, 0 for none.  Under a limit the second pool holds no freed blocks.
     void set_budget(uint64_t bytes);
     // Allocation on stream `st`, with budget accounting.

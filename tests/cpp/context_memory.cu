@@ -97,17 +97,17 @@ static void budget() {
     cpvs::Ctx c;
     begin(c);
     void* p = nullptr;
-    check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(nullptr)) == CPVS_OK, "an index without a budget");
+    check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(64 * MiB, nullptr)) == CPVS_OK, "an index without a budget");
     c.release(p, 64 * MiB, true, nullptr);
     void* held = nullptr;
-    check(c.alloc(&held, 64 * MiB, true, nullptr, c.index_source(nullptr)) == CPVS_OK, "an index without a budget");
+    check(c.alloc(&held, 64 * MiB, true, nullptr, c.index_source(64 * MiB, nullptr)) == CPVS_OK, "an index without a budget");
     c.set_budget(200 * MiB);
-    check(c.index_source(nullptr) == nullptr, "an index under a budget comes from the context's pool");
+    check(c.index_source(64 * MiB, nullptr) == nullptr, "an index under a budget comes from the context's pool");
     check(model::reserved() == 64 * MiB, "freed blocks of the second pool go back with a budget");
     c.release(held, 64 * MiB, true, nullptr);
     check(model::reserved() == 0, "blocks of the second pool freed under a budget go back");
     for (int k = 0; k < 4; ++k) {
-        check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(nullptr)) == CPVS_OK, "an index under a budget");
+        check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(64 * MiB, nullptr)) == CPVS_OK, "an index under a budget");
         c.release(p, 64 * MiB, true, nullptr);
         check(c.alloc(&p, 200 * MiB, true, nullptr) == CPVS_OK, "the whole budget");
         c.release(p, 200 * MiB, true, nullptr);
@@ -120,7 +120,7 @@ static void full() {
     cpvs::Ctx c;
     begin(c);
     void *p = nullptr, *q = nullptr;
-    cudaMemPool_t second = c.index_source(nullptr);
+    cudaMemPool_t second = c.index_source(64 * MiB, nullptr);
     check(second != nullptr, "a second pool");
     check(c.alloc(&p, 1000 * MiB, false, nullptr) == CPVS_OK, "a large scratch");
     c.release(p, 1000 * MiB, false, nullptr);
@@ -131,10 +131,26 @@ static void full() {
     c.release(p, 1000 * MiB, false, nullptr);
 }
 
+// The second pool is made for the first large index alone.
+static void pool_when_needed() {
+    cpvs::Ctx c;
+    begin(c);
+    for (uint64_t b = 1 << 10; b <= 8 * MiB; b *= 8)
+        check(c.index_source(b, nullptr) == nullptr, "a small index comes from the context's pool");
+    model::capturing = true;
+    check(c.index_source(64 * MiB, nullptr) == nullptr && !c.index_beyond_rule(nullptr), "no pool during a capture");
+    model::capturing = false;
+    check(model::pools.size() == 1, "no pool before it is needed");
+    check(c.index_source(64 * MiB, nullptr) != nullptr && c.index_beyond_rule(nullptr), "a pool for a large index");
+    check(c.index_source(64 * MiB, nullptr) == c.index_pool && model::pools.size() == 2, "one such pool");
+    check(c.index_source(8 * MiB, nullptr) == nullptr, "still none for a small index");
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "budget") budget();
     else if (what == "full") full();
+    else if (what == "pool_when_needed") pool_when_needed();
     else return 2;
     std::printf("ok\n");
     return 0;

@@ -18,7 +18,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["budget", "full"])
+@pytest.mark.parametrize("what", ["budget", "full", "pool_when_needed"])
 def test_context_memory(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
