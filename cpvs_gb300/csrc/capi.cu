@@ -184,7 +184,8 @@ cpvs_status build_into_shadows(cpvs_ctx* ctx, const std::vector<cpvs::SourceSpec
 // later ones.  2^26 points, an 8192^2 map (first / later): 495 -> 441 / 466 ->
 // 393 us with 8 levels for 7; 2^25, a 2048^2 map of 45 objects: 231 -> 189 / 215
 // -> 156; 1.3 * 2^22 of them: 55 -> 49 / 45 -> 38; a cell per point gained nothing
-// more at 1.3 * 2^18 and lost 3% of the first lookup at 2^24.
+// more at 1.3 * 2^18 and lost 3% of the first lookup at 2^24.  Such grids, for
+// they stay as long as their shadows, are at most kIndexBeyond bytes in all.
 constexpr uint32_t kTopFactor = 8;
 void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor = kTopFactor,
                  uint64_t points = 0) {
@@ -198,6 +199,7 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
         const int least = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, 0);
         int depth = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, points / 2);
         auto bytes = [&] { return uint64_t(4) << (3 * depth); };
+        while (depth > least && c.index_beyond + bytes() > cpvs::Ctx::kIndexBeyond) --depth;
         while (depth > 0 && c.alloc((void**)&s->top, bytes(), true, st,
                                     depth > least ? c.index_source(bytes(), st) : nullptr) != CPVS_OK) {
             s->top = nullptr;
@@ -210,6 +212,8 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
         }
         s->top_bytes = bytes();
         s->top_depth = depth;
+        s->top_beyond = depth > least ? s->top_bytes : 0;
+        c.index_beyond += s->top_beyond;
         grids.push_back(cpvs::TopGrid{s->dag, s->words, depth, s->top});
         owners.push_back(s);
     }
@@ -218,9 +222,11 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
     if (cpvs::launch_top_index(grids.data(), grids.size(), st) != CPVS_OK) {
         for (cpvs_shadow* s : owners) {
             s->ctx->c.release(s->top, s->top_bytes, true, st);
+            s->ctx->c.index_beyond -= s->top_beyond;
             s->top = nullptr;
             s->top_bytes = ~0ull;
             s->top_depth = 0;
+            s->top_beyond = 0;
         }
         cudaGetLastError();
         return;
@@ -760,6 +766,7 @@ void cpvs_shadow_destroy(cpvs_shadow* s) {
     if (!s) return;
     cudaSetDevice(s->ctx->c.device);
     if (s->top) s->ctx->c.release(s->top, s->top_bytes, true, nullptr, s->last_use());
+    s->ctx->c.index_beyond -= s->top_beyond;
     block_unref(s->block, s->last_use());
     delete s;
 }

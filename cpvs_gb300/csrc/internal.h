@@ -327,6 +327,9 @@ struct Ctx {
     // Whether a top grid may be larger than the DAG's size allows (no budget, no
     // capture on `st`).
     bool index_beyond_rule(cudaStream_t st) const;
+    // The bytes of such grids that there are, and the most of them.
+    static constexpr uint64_t kIndexBeyond = 1ull << 30;
+    uint64_t index_beyond = 0;
     // The limit, 0 for none.  Under a limit the second pool holds no freed blocks.
     void set_budget(uint64_t bytes);
     // Allocation on stream `st`, with budget accounting.

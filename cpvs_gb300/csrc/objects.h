@@ -118,6 +118,7 @@ struct cpvs_shadow : DeviceObject {
     uint32_t* top = nullptr;   // dense top index for lookups, built on the first lookup
     uint64_t top_bytes = 0;
     int top_depth = 0;         // levels below the root that `top` resolves
+    uint64_t top_beyond = 0;   // top_bytes where they are more than the DAG's size allows, else 0
     uint32_t num_levels = 0;
     bool leafmasks = false;
     uint32_t root_mask = 0;
