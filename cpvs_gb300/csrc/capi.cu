@@ -187,8 +187,9 @@ cpvs_status build_into_shadows(cpvs_ctx* ctx, const std::vector<cpvs::SourceSpec
 // more at 1.3 * 2^18 and lost 3% of the first lookup at 2^24.  Such grids, for
 // they stay as long as their shadows, are at most kIndexBeyond bytes in all.
 constexpr uint32_t kTopFactor = 8;
-void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor = kTopFactor,
-                 uint64_t points = 0) {
+void make_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor,
+               uint64_t points) {
+    std::lock_guard<std::mutex> lock(shadows[0]->ctx->c.index_mutex);
     std::vector<cpvs::TopGrid> grids;
     std::vector<cpvs_shadow*> owners;
     for (size_t i = 0; i < count; ++i) {
@@ -231,10 +232,16 @@ void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t s
         cudaGetLastError();
         return;
     }
-    DeviceObject::touch_all(owners.data(), owners.size(), st);
+    DeviceObject::indexed_all(owners.data(), owners.size(), st);
+}
+// Indices for the shadows (of one context), and `st` after their making.
+void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor = kTopFactor,
+                 uint64_t points = 0) {
+    make_tops(shadows, count, st, max_factor, points);
+    DeviceObject::await_indices(shadows, count, st);
 }
 void ensure_top(const cpvs_shadow* s, cudaStream_t st, uint32_t max_factor = kTopFactor, uint64_t points = 0) {
-    if (!s->top && s->top_bytes != ~0ull) ensure_tops(&s, 1, st, max_factor, points);
+    ensure_tops(&s, 1, st, max_factor, points);
 }
 
 }  // namespace
@@ -1093,8 +1100,9 @@ cpvs_status cpvs_grid_words(const cpvs_grid* g, uint32_t* dag_out, uint64_t dag_
 }
 
 // The grid's top index, built on its first lookup (stream-ordered).
-static void ensure_grid_top(const cpvs_grid* cg, cudaStream_t st) {
+static void make_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     cpvs_grid* g = const_cast<cpvs_grid*>(cg);
+    std::lock_guard<std::mutex> lock(g->ctx->c.index_mutex);
     if (g->gtop || g->gtop_bytes == ~0ull) return;
     const int depth = cpvs::grid_top_depth(g->length, g->dag_levels, g->leafmasks, g->words);
     const uint64_t bytes = uint64_t(4) << (3 * (cpvs::log2_u32(g->length) + depth));
@@ -1110,6 +1118,11 @@ static void ensure_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     }
     g->gtop_bytes = bytes;
     g->gtop_depth = depth;
+    DeviceObject::indexed_all(&g, 1, st);
+}
+static void ensure_grid_top(const cpvs_grid* g, cudaStream_t st) {
+    make_grid_top(g, st);
+    DeviceObject::await_indices(&g, 1, st);
 }
 
 cpvs_status cpvs_grid_lookup_ndc(const cpvs_grid* g, const float* xyz, uint64_t n, uint32_t* bits_out, uint32_t flags,

@@ -27,12 +27,13 @@ struct DeviceObject {
     DeviceObject& operator=(const DeviceObject&) = delete;
     ~DeviceObject() {
         std::lock_guard<std::mutex> lock(c_->event_mutex);
-        drop();
+        drop(use_);
+        drop(index_);
     }
     void touch(cudaStream_t st) const {
         std::lock_guard<std::mutex> lock(c_->event_mutex);
         if (!use_ || use_->refs > 1) {
-            drop();
+            drop(use_);
             use_ = new UseEvent{c_->take_event(), 1u};
         }
         if (use_->event) cudaEventRecord(use_->event, st);
@@ -42,6 +43,41 @@ struct DeviceObject {
     // their own, from that context's pool and under its mutex.
     template <class T>
     static void touch_all(T* const* objects, size_t count, cudaStream_t st) {
+        record_all(objects, count, st, false);
+    }
+    // touch_all after `st` was given the work that makes the objects' indices:
+    // until it is done, the uses of an index on other streams wait for it.
+    template <class T>
+    static void indexed_all(T* const* objects, size_t count, cudaStream_t st) {
+        record_all(objects, count, st, true);
+    }
+    // Before a use of the indices of `objects` (of one context) on `st`.  (A
+    // capturing stream takes no wait for work outside its capture: what it
+    // records runs later.)
+    template <class T>
+    static void await_indices(T* const* objects, size_t count, cudaStream_t st) {
+        if (!count) return;
+        std::lock_guard<std::mutex> lock(objects[0]->c_->event_mutex);
+        for (size_t i = 0; i < count; ++i) {
+            const DeviceObject& o = *objects[i];
+            if (!o.index_ || st == o.index_stream_ || !o.index_->event) continue;
+            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+                cudaGetLastError();
+                return;
+            }
+            if (cudaEventQuery(o.index_->event) == cudaSuccess) {
+                o.drop(o.index_);
+                continue;
+            }
+            cudaGetLastError();  // (not ready)
+            cudaStreamWaitEvent(st, o.index_->event, 0);
+        }
+    }
+
+private:
+    template <class T>
+    static void record_all(T* const* objects, size_t count, cudaStream_t st, bool index) {
         if (!count) return;
         cpvs::Ctx* c = objects[0]->c_;
         uint32_t mine = 0;
@@ -52,29 +88,37 @@ struct DeviceObject {
                 objects[i]->touch(st);
         }
         std::lock_guard<std::mutex> lock(c->event_mutex);
-        auto* u = new UseEvent{c->take_event(), mine};
+        auto* u = new UseEvent{c->take_event(), index ? 2 * mine : mine};
         if (u->event) cudaEventRecord(u->event, st);
         for (size_t i = 0; i < count; ++i) {
             if (objects[i]->c_ != c) continue;
-            objects[i]->drop();
+            objects[i]->drop(objects[i]->use_);
             objects[i]->use_ = u;
+            if (!index) continue;
+            objects[i]->drop(objects[i]->index_);
+            objects[i]->index_ = u;
+            objects[i]->index_stream_ = st;
         }
     }
+
+public:
     cudaEvent_t last_use() const {
         std::lock_guard<std::mutex> lock(c_->event_mutex);
         return use_ ? use_->event : nullptr;
     }
 
 private:
-    void drop() const {
-        if (use_ && --use_->refs == 0) {
-            c_->give_event(use_->event);
-            delete use_;
+    void drop(UseEvent*& u) const {
+        if (u && --u->refs == 0) {
+            c_->give_event(u->event);
+            delete u;
         }
-        use_ = nullptr;
+        u = nullptr;
     }
     cpvs::Ctx* c_;
     mutable UseEvent* use_ = nullptr;
+    mutable UseEvent* index_ = nullptr;  // after the object's index, until that is known to be done
+    mutable cudaStream_t index_stream_ = nullptr;
 };
 
 struct cpvs_hierarchy : DeviceObject {
