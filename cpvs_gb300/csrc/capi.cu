@@ -195,14 +195,17 @@ void make_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st,
     for (size_t i = 0; i < count; ++i) {
         cpvs_shadow* s = const_cast<cpvs_shadow*>(shadows[i]);
         if (s->top || s->top_bytes == ~0ull) continue;
+        // none in a recorded graph, whose memory and work are there when the
+        // graph runs and not before: the recorded lookups do without
+        if (owners.empty() && cpvs::capturing(st)) return;
         cpvs::Ctx& c = s->ctx->c;
-        if (points && !c.index_beyond_rule(st)) points = 0;
+        if (c.budget) points = 0;
         const int least = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, 0);
         int depth = cpvs::top_index_depth(s->num_levels, s->leafmasks, s->words, max_factor, points / 2);
         auto bytes = [&] { return uint64_t(4) << (3 * depth); };
         while (depth > least && c.index_beyond + bytes() > cpvs::Ctx::kIndexBeyond) --depth;
         while (depth > 0 && c.alloc((void**)&s->top, bytes(), true, st,
-                                    depth > least ? c.index_source(bytes(), st) : nullptr) != CPVS_OK) {
+                                    depth > least ? c.index_source(bytes()) : nullptr) != CPVS_OK) {
             s->top = nullptr;
             cudaGetLastError();
             depth = depth > least ? least : 0;
@@ -267,6 +270,7 @@ int lookup_qpt(const cpvs_shadow* s, const void* q, bool ndc, bool host_in, uint
     cpvs::Ctx& c = s->ctx->c;
     if (c.lookup_qpt) return c.lookup_qpt;
     int& t = c.lookup_qpt_tuned[s->num_levels % CPVS_MAX_LEVELS][ndc ? 1 : 0][host_in ? 1 : 0];
+    if (!t && cpvs::capturing(st)) return 2;  // (a recorded launch has no time; not kept)
     if (!t)
         t = cpvs::tune_lookup(s->dag, s->words, s->num_levels, s->leafmasks, s->top, s->top_depth, q, ndc, n, bits, st);
     return t;
@@ -1103,11 +1107,11 @@ cpvs_status cpvs_grid_words(const cpvs_grid* g, uint32_t* dag_out, uint64_t dag_
 static void make_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     cpvs_grid* g = const_cast<cpvs_grid*>(cg);
     std::lock_guard<std::mutex> lock(g->ctx->c.index_mutex);
-    if (g->gtop || g->gtop_bytes == ~0ull) return;
+    if (g->gtop || g->gtop_bytes == ~0ull || cpvs::capturing(st)) return;  // (as a shadow's)
     const int depth = cpvs::grid_top_depth(g->length, g->dag_levels, g->leafmasks, g->words);
     const uint64_t bytes = uint64_t(4) << (3 * (cpvs::log2_u32(g->length) + depth));
     if (depth <= 0 ||
-        g->ctx->c.alloc((void**)&g->gtop, bytes, true, st, g->ctx->c.index_source(bytes, st)) != CPVS_OK ||
+        g->ctx->c.alloc((void**)&g->gtop, bytes, true, st, g->ctx->c.index_source(bytes)) != CPVS_OK ||
         cpvs::launch_grid_top_index(g->dag, g->words, g->cell_words, g->length, g->dag_levels, depth, g->gtop, st) !=
             CPVS_OK) {
         if (g->gtop) g->ctx->c.release(g->gtop, bytes, true, st);

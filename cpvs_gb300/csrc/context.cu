@@ -75,18 +75,15 @@ void Ctx::release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cud
 constexpr uint64_t kIndexOwn = 16ull << 20;
 constexpr uint64_t kIndexKeep = 1ull << 30;  // 16 of the largest
 
-bool Ctx::index_beyond_rule(cudaStream_t st) const {
-    if (budget) return false;
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return capturing == cudaStreamCaptureStatusNone;
+bool capturing(cudaStream_t st) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
 }
 
-cudaMemPool_t Ctx::index_source(uint64_t bytes, cudaStream_t st) {
-    if (bytes < kIndexOwn || !index_beyond_rule(st)) return nullptr;
+cudaMemPool_t Ctx::index_source(uint64_t bytes) {
+    if (bytes < kIndexOwn || budget) return nullptr;
     if (!index_pool && create_pool(device, &index_pool, kIndexKeep) != cudaSuccess) {
         cudaGetLastError();
         index_pool = nullptr;

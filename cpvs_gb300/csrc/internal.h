@@ -275,6 +275,9 @@ struct KernelTimer {
 // A pool that holds on to `keep` bytes, freed blocks included, before it returns
 // any to the CUDA driver.
 cudaError_t create_pool(int device, cudaMemPool_t* pool, uint64_t keep);
+// Whether `st` is recording a graph (or may be: a legacy stream beside one
+// that is).
+bool capturing(cudaStream_t st);
 
 struct Ctx {
     Timing timing;
@@ -323,11 +326,9 @@ struct Ctx {
     // memory cost a context's first lookup 150 to 250 us (first frame of a
     // 1024^2 map 820 -> 1065 us, filtered 2048^2 628 -> 808).  Under a budget
     // none: the pool would hold its freed blocks beside the budget's.
-    cudaMemPool_t index_source(uint64_t bytes, cudaStream_t st);
-    // Whether a top grid may be larger than the DAG's size allows (no budget, no
-    // capture on `st`).
-    bool index_beyond_rule(cudaStream_t st) const;
-    // The bytes of such grids that there are, and the most of them.
+    cudaMemPool_t index_source(uint64_t bytes);
+    // The bytes of top grids larger than their DAG's size allows (without a
+    // budget) that there are, and the most of them.
     static constexpr uint64_t kIndexBeyond = 1ull << 30;
     uint64_t index_beyond = 0;
     // Held while an object's index is made: lookups of several host threads may

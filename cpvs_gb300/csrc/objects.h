@@ -61,11 +61,7 @@ struct DeviceObject {
         for (size_t i = 0; i < count; ++i) {
             const DeviceObject& o = *objects[i];
             if (!o.index_ || st == o.index_stream_ || !o.index_->event) continue;
-            cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
-                cudaGetLastError();
-                return;
-            }
+            if (cpvs::capturing(st)) return;
             if (cudaEventQuery(o.index_->event) == cudaSuccess) {
                 o.drop(o.index_);
                 continue;

@@ -19,7 +19,6 @@ struct Pool {
 };
 std::vector<Pool*> pools;
 std::map<void*, std::pair<Pool*, uint64_t>> blocks;
-bool capturing = false;
 char place[1 << 12];
 size_t next = 0;
 
@@ -60,7 +59,7 @@ cudaError_t release(void* p, cudaStream_t) {
     return cudaSuccess;
 }
 cudaError_t is_capturing(cudaStream_t, cudaStreamCaptureStatus* s) {
-    *s = capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
+    *s = cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
 cudaError_t ok() { return cudaSuccess; }
@@ -97,17 +96,17 @@ static void budget() {
     cpvs::Ctx c;
     begin(c);
     void* p = nullptr;
-    check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(64 * MiB, nullptr)) == CPVS_OK, "an index without a budget");
+    check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(64 * MiB)) == CPVS_OK, "an index without a budget");
     c.release(p, 64 * MiB, true, nullptr);
     void* held = nullptr;
-    check(c.alloc(&held, 64 * MiB, true, nullptr, c.index_source(64 * MiB, nullptr)) == CPVS_OK, "an index without a budget");
+    check(c.alloc(&held, 64 * MiB, true, nullptr, c.index_source(64 * MiB)) == CPVS_OK, "an index without a budget");
     c.set_budget(200 * MiB);
-    check(c.index_source(64 * MiB, nullptr) == nullptr, "an index under a budget comes from the context's pool");
+    check(c.index_source(64 * MiB) == nullptr, "an index under a budget comes from the context's pool");
     check(model::reserved() == 64 * MiB, "freed blocks of the second pool go back with a budget");
     c.release(held, 64 * MiB, true, nullptr);
     check(model::reserved() == 0, "blocks of the second pool freed under a budget go back");
     for (int k = 0; k < 4; ++k) {
-        check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(64 * MiB, nullptr)) == CPVS_OK, "an index under a budget");
+        check(c.alloc(&p, 64 * MiB, true, nullptr, c.index_source(64 * MiB)) == CPVS_OK, "an index under a budget");
         c.release(p, 64 * MiB, true, nullptr);
         check(c.alloc(&p, 200 * MiB, true, nullptr) == CPVS_OK, "the whole budget");
         c.release(p, 200 * MiB, true, nullptr);
@@ -120,7 +119,7 @@ static void full() {
     cpvs::Ctx c;
     begin(c);
     void *p = nullptr, *q = nullptr;
-    cudaMemPool_t second = c.index_source(64 * MiB, nullptr);
+    cudaMemPool_t second = c.index_source(64 * MiB);
     check(second != nullptr, "a second pool");
     check(c.alloc(&p, 1000 * MiB, false, nullptr) == CPVS_OK, "a large scratch");
     c.release(p, 1000 * MiB, false, nullptr);
@@ -136,14 +135,11 @@ static void pool_when_needed() {
     cpvs::Ctx c;
     begin(c);
     for (uint64_t b = 1 << 10; b <= 8 * MiB; b *= 8)
-        check(c.index_source(b, nullptr) == nullptr, "a small index comes from the context's pool");
-    model::capturing = true;
-    check(c.index_source(64 * MiB, nullptr) == nullptr && !c.index_beyond_rule(nullptr), "no pool during a capture");
-    model::capturing = false;
+        check(c.index_source(b) == nullptr, "a small index comes from the context's pool");
     check(model::pools.size() == 1, "no pool before it is needed");
-    check(c.index_source(64 * MiB, nullptr) != nullptr && c.index_beyond_rule(nullptr), "a pool for a large index");
-    check(c.index_source(64 * MiB, nullptr) == c.index_pool && model::pools.size() == 2, "one such pool");
-    check(c.index_source(8 * MiB, nullptr) == nullptr, "still none for a small index");
+    check(c.index_source(64 * MiB) != nullptr, "a pool for a large index");
+    check(c.index_source(64 * MiB) == c.index_pool && model::pools.size() == 2, "one such pool");
+    check(c.index_source(8 * MiB) == nullptr, "still none for a small index");
 }
 
 int main(int argc, char** argv) {
