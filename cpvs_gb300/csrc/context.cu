@@ -59,10 +59,14 @@ void Ctx::give_event(cudaEvent_t e) {
         cudaEventDestroy(e);
 }
 
+void Ctx::await_use(cudaEvent_t last_use) {
+    if (last_use && cudaStreamWaitEvent(free_stream, last_use, 0) != cudaSuccess) cudaGetLastError();
+}
+
 void Ctx::release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cudaEvent_t last_use) {
     if (persistent) {
         if (p) {
-            if (last_use) cudaStreamWaitEvent(free_stream, last_use, 0);
+            await_use(last_use);
             cudaFreeAsync(p, free_stream);
         }
         in_use -= std::min(in_use, bytes);

@@ -338,6 +338,10 @@ struct Ctx {
     void set_budget(uint64_t bytes);
     // Allocation on stream `st`, with budget accounting.
     cpvs_status alloc(void** p, uint64_t bytes, bool persistent, cudaStream_t st, cudaMemPool_t from = nullptr);
+    // What is freed from here on is so after `last_use` is reached.  (A use
+    // recorded in a capture can't be waited for: its graph runs when the caller
+    // has it run, and before the object is destroyed.)
+    void await_use(cudaEvent_t last_use);
     // Scratch: freed in the order of `st`.  Persistent: freed once
     // `last_use` (the last event recorded after work on the block) is reached.
     void release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cudaEvent_t last_use = nullptr);

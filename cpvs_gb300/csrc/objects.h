@@ -142,7 +142,7 @@ struct DagBlock {
 inline void block_unref(DagBlock* b, cudaEvent_t last_use) {
     if (!b) return;
     cpvs::Ctx& c = b->ctx->c;
-    if (last_use) cudaStreamWaitEvent(c.free_stream, last_use, 0);  // the free waits for every holder
+    c.await_use(last_use);  // the free waits for every holder
     if (--b->refs == 0) {
         c.release(b->base, b->bytes, true, nullptr, nullptr);
         delete b;

@@ -76,3 +76,32 @@ def test_first_lookup_in_a_graph(cp, oracle, kind):
         eager.zero_()
         run(None, eager)
         assert same(eager)
+
+
+@pytest.mark.gpu
+def test_objects_used_in_a_graph_are_destroyed(cp, oracle):
+    """An object whose last use was recorded in a capture: its release waits for
+    nothing of the capture and leaves no error behind for the next call."""
+    import torch
+    n = 256
+    d = scene.rasterise(scene.make_scene(n, 0.9, 20, 4, seed=2))
+    want = oracle.build(d).dag
+    q = scene.ndc_queries_mixed(d, 1 << 12, 5)
+    pts = torch.from_numpy(q).cuda()
+    out = torch.zeros(len(q) // 32, dtype=torch.int32, device="cuda")
+    ctx = cp.Context(0)
+    ids = torch.zeros(len(q), dtype=torch.int32, device="cuda")
+    for trial in range(3):
+        sh = cp.CompressedShadow.from_depth(d, ctx=ctx)
+        sh.lookup_ndc(pts)
+        torch.cuda.synchronize()
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            sh.lookup_ndc(pts, out=out, stream=stream)
+            cp.lookup_ndc_multi([sh], ids, pts, out=out, stream=stream)
+        graph.replay()
+        torch.cuda.synchronize()
+        del graph, sh
+        again = cp.CompressedShadow.from_depth(d, ctx=ctx)
+        assert np.array_equal(again.get_dag(), want)
+        del again
