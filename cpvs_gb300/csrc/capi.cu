@@ -261,19 +261,17 @@ MultiDag shadow_table_entry(const cpvs_shadow* s) {
 namespace {
 
 // Queries per thread for a lookup on `s`: the context's fixed choice, or the
-// tuned one for this DAG depth and input kind (tuned on the first batch that
-// needs it).  Points read in place from host memory cross the host link with
-// its latency, which favours more queries in flight per thread than points
-// in device memory do, so the two kinds are tuned apart.
+// tuned one for such lookups (tuned on the first batch that needs it), or one
+// where there is nothing to tune.
 int lookup_qpt(const cpvs_shadow* s, const void* q, bool ndc, bool host_in, uint64_t n, uint32_t* bits,
                cudaStream_t st) {
     cpvs::Ctx& c = s->ctx->c;
     if (c.lookup_qpt) return c.lookup_qpt;
-    int& t = c.lookup_qpt_tuned[s->num_levels % CPVS_MAX_LEVELS][ndc ? 1 : 0][host_in ? 1 : 0];
-    if (!t && cpvs::capturing(st)) return 2;  // (a recorded launch has no time; not kept)
-    if (!t)
-        t = cpvs::tune_lookup(s->dag, s->words, s->num_levels, s->leafmasks, s->top, s->top_depth, q, ndc, n, bits, st);
-    return t;
+    int* t = c.lookup_choice(s->num_levels, s->top ? s->top_depth : 0, s->leafmasks, ndc, host_in, n);
+    if (!t || (!*t && cpvs::capturing(st))) return 1;  // (a recorded launch has no time)
+    if (!*t)
+        *t = cpvs::tune_lookup(s->dag, s->words, s->num_levels, s->leafmasks, s->top, s->top_depth, q, ndc, n, bits, st);
+    return *t;
 }
 
 }  // namespace

@@ -79,6 +79,11 @@ void Ctx::release(void* p, uint64_t bytes, bool persistent, cudaStream_t st, cud
 constexpr uint64_t kIndexOwn = 16ull << 20;
 constexpr uint64_t kIndexKeep = 1ull << 30;  // 16 of the largest
 
+int* Ctx::lookup_choice(uint32_t num_levels, int depth, bool leafmasks, bool ndc, bool host_in, uint64_t n) {
+    if (n < std::max(num_sms, 1) * 2048ull) return nullptr;  // 2048 threads to an SM
+    return &lookup_qpt_tuned[num_levels % CPVS_MAX_LEVELS][std::min(depth, kTopIndexDepth)][leafmasks][ndc][host_in];
+}
+
 bool capturing(cudaStream_t st) {
     cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;

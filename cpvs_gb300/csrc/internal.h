@@ -286,9 +286,19 @@ struct Ctx {
     int cluster_blocks = -1;  // blocks per cluster of the small-level build kernels (-1: not probed yet)
     bool pageable_access = false;  // the GPU reads pageable host memory in place
     // lookup queries per thread: fixed by cpvs_ctx_set_option, else tuned
-    // once per (DAG levels, NDC or voxel input)
+    // once per kind of lookup
     int lookup_qpt = 0;
-    int lookup_qpt_tuned[CPVS_MAX_LEVELS][2][2] = {};  // [levels][ndc][points in host memory]
+    int lookup_qpt_tuned[CPVS_MAX_LEVELS][kTopIndexDepth + 1][2][2][2] = {};
+    // Where the tuned number of such lookups is kept (0: not tuned yet); null:
+    // one query a thread, without timing.  The levels that the index leaves to
+    // the descent set the work, and the index's depth varies with a DAG's first
+    // batch.  Points read in place from host memory cross the host link with its
+    // latency, which favours more queries in flight per thread than points in
+    // device memory do.  Batches whose queries are all in flight at once with
+    // one a thread have nothing to gain from more, and take less than a timing's
+    // noise: 500 to 2^18 points, maps of 256^2 to 8192^2, 2.0 to 4.7 us with one
+    // query a thread, 2.6 to 5.6 with two, 3.5 to 6.5 with four.
+    int* lookup_choice(uint32_t num_levels, int depth, bool leafmasks, bool ndc, bool host_in, uint64_t n);
     // build launch shapes fixed by cpvs_ctx_set_option (0: timed per plan on
     // its first build): the largest level the cluster kernels take, and the
     // inner-level insert's grid in resident waves

@@ -1,4 +1,4 @@
-// A context's memory over its two pools (csrc/context.cu), with a model of the
+// A context's memory over its two pools, and its choices (csrc/context.cu), with a model of the
 // CUDA pools in place of the driver's: a device of `capacity` bytes, pools that
 // reserve what they hand out and keep what is freed up to their threshold.
 #include <cuda_runtime.h>
@@ -142,11 +142,28 @@ static void pool_when_needed() {
     check(c.index_source(8 * MiB) == nullptr, "still none for a small index");
 }
 
+// A lookup's tuned variant is kept by what sets its work, and not for batches
+// too small to time.
+static void lookup_choice() {
+    cpvs::Ctx c;
+    c.num_sms = 152;
+    std::map<int*, int> places;
+    for (uint32_t levels = 2; levels <= 17; ++levels)
+        for (int depth = 0; depth <= 8; ++depth)
+            for (int k = 0; k < 8; ++k) {
+                check(!c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 500), "a small batch is not timed");
+                check(!c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 1 << 18), "a small batch is not timed");
+                ++places[c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 1 << 20)];
+            }
+    check(places.size() == 16 * 9 * 8 && !places.count(nullptr), "a place for every kind");
+}
+
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "budget") budget();
     else if (what == "full") full();
     else if (what == "pool_when_needed") pool_when_needed();
+    else if (what == "lookup_choice") lookup_choice();
     else return 2;
     std::printf("ok\n");
     return 0;

@@ -1,5 +1,5 @@
-"""A context's memory over its two pools (tests/cpp/context_memory.cu, host code
-over a model of the CUDA pools)."""
+"""A context's memory over its two pools, and its choices
+(tests/cpp/context_memory.cu, host code over a model of the CUDA pools)."""
 import os
 import subprocess
 
@@ -18,7 +18,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["budget", "full", "pool_when_needed"])
+@pytest.mark.parametrize("what", ["budget", "full", "pool_when_needed", "lookup_choice"])
 def test_context_memory(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr
