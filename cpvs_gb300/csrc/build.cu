@@ -669,6 +669,8 @@ struct LeafColumns {
     unsigned int* heavy_ctr;    // [0] and [1]: their counts (zeroed per build)
     unsigned int* any_nan;      // nonzero: some map holds a NaN, or may (zeroed per build)
     uint32_t* kept;             // one bit per leaf: first occurrence of its class (zeroed per build)
+    uint32_t* err;              // the errors of the column and class passes, which run beside the clearing of the
+                                // build's error word (zeroed per build before them; k_layout joins the two)
 };
 
 // A column's record: its first run entry, that run's class, the run's first
@@ -699,7 +701,7 @@ __device__ __forceinline__ uint32_t full_run_end(float v, float s, uint32_t zmax
 // entry index by the column pass, an earlier kernel, so a slot's claimant is
 // compared straight from memory (no publication order to keep).
 __device__ __forceinline__ uint32_t leaf_class_insert(const LeafColumns& lc, uint64_t h, uint32_t j,
-                                                      const uint64_t M[8], uint32_t cid, uint32_t* err) {
+                                                      const uint64_t M[8], uint32_t cid) {
     const unsigned long long key = (h & 0xFFFFFFFF00000000ull) | cid;
     uint64_t s = h & lc.table_mask;
     for (uint64_t probe = 0; probe <= lc.table_mask; ++probe) {
@@ -724,19 +726,19 @@ __device__ __forceinline__ uint32_t leaf_class_insert(const LeafColumns& lc, uin
         }
         s = (s + 1) & lc.table_mask;
     }
-    atomicOr(err, 16u);  // table full: the result is void, reported (the plan grows)
+    atomicOr(lc.err, 16u);  // table full: the result is void, reported (the plan grows)
     return cid;
 }
 
 // One thread per non-uniform run: its class id into the run entry.
-__global__ void __launch_bounds__(kThreads) k_leaf_classes(LeafColumns lc, uint32_t* err) {
+__global__ void __launch_bounds__(kThreads) k_leaf_classes(LeafColumns lc) {
     chain_enter();
     const uint32_t np = *lc.pending_ctr;
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) {
         const uint2 pe = lc.pending[p];
         const uint32_t cid = pe.x;
         if (cid >= lc.run_cap) {
-            atomicOr(err, 512u);
+            atomicOr(lc.err, 512u);
             continue;
         }
         const ulonglong2* o = reinterpret_cast<const ulonglong2*>(lc.cls_slices + (size_t)cid * 8);
@@ -748,7 +750,7 @@ __global__ void __launch_bounds__(kThreads) k_leaf_classes(LeafColumns lc, uint3
             M[2 * q + 1] = t.y;
         }
         const uint32_t j = lc.cls_job[cid];
-        const uint32_t id = leaf_class_insert(lc, leaf_hash(j, M), j, M, cid, err);
+        const uint32_t id = leaf_class_insert(lc, leaf_hash(j, M), j, M, cid);
         lc.runs[cid].y = id;
         if (pe.y) lc.colrec[pe.y - 1u].y = id;  // its column's first run
     }
@@ -877,7 +879,7 @@ constexpr uint32_t kColChunk = kThreads;
 constexpr uint32_t kSteepCells = 16;  // leaf cells from which a column is queued in front
 
 template <bool POW2>
-__global__ void __launch_bounds__(kThreads) k_leaf_columns(LeafColumns lc, uint32_t* err) {
+__global__ void __launch_bounds__(kThreads) k_leaf_columns(LeafColumns lc) {
     chain_enter();
     __shared__ uint32_t sm[32];
     __shared__ uint32_t s_base, s_at[2], s_queue[2][kThreads / 32];
@@ -912,7 +914,7 @@ __global__ void __launch_bounds__(kThreads) k_leaf_columns(LeafColumns lc, uint3
         __syncthreads();
         const uint32_t off = s_base + pre;
         const bool fits = (uint64_t)s_base + tot <= lc.run_cap;
-        if (!fits && threadIdx.x == 0) atomicOr(err, 1u);  // more runs than the plan holds: reported, the plan grows
+        if (!fits && threadIdx.x == 0) atomicOr(lc.err, 1u);  // more runs than the plan holds: reported, the plan grows
         bool queue = false;
         uint32_t k = 0, zc = 0, nrun = 0;
         if (q < ncols) {
@@ -2891,13 +2893,18 @@ struct JobLayout {
 
 // With `root_mask` (and `lvt`), also the root mask of every job (the first
 // word of its DAG).
+// With `leaf_err`, the leaf branch's errors join those at `err`.
 // With `host` (mapped host memory), the `bytes16` 16-byte words of the results
 // at `res` are then written there and `*ready` is set: the host polls it
 // instead of waiting for a copy and the stream.
 __global__ void k_layout(SegDev seg, JobLayout lay, const uint32_t* __restrict__ root_level, uint32_t njobs, int bottom,
-                         const LevelDev* __restrict__ lvt, uint32_t* root_mask, const uint4* res, uint4* host,
-                         uint32_t bytes16, uint32_t* ready) {
+                         const LevelDev* __restrict__ lvt, uint32_t* root_mask, const uint32_t* leaf_err, uint32_t* err,
+                         const uint4* res, uint4* host, uint32_t bytes16, uint32_t* ready) {
     chain_enter();
+    if (leaf_err && threadIdx.x == 0) {
+        const uint32_t e = __ldcg(leaf_err);
+        if (e) atomicOr(err, e);
+    }
     // single block: each thread sums its jobs, then a block scan over jobs in
     // rounds of blockDim
     __shared__ uint32_t sm[64];
@@ -3188,7 +3195,8 @@ struct BuildPlan {
     LeafGroupDev* groups_dev = nullptr;
     uint2* ztiles_dev = nullptr;
     uint32_t* lmeta = nullptr;  // [0] groups, [1] columns; zeroed per build: [4] run entries reserved,
-                                // [5] pending runs, [6], [7] queued columns, [8] a map may hold a NaN
+                                // [5] pending runs, [6], [7] queued columns, [8] a map may hold a NaN,
+                                // [9] the column and class passes' errors
     uint32_t* ltiles = nullptr;  // level 3's tiles: leaves, then first leaves
     uint32_t* lkept = nullptr;   // one bit per leaf (cap[2])
     uint32_t leaf_steps = 1;     // kLeafTile level-3 nodes a block of k_leaf_count takes, times this
@@ -3209,7 +3217,7 @@ struct BuildPlan {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t done = nullptr;  // recorded after the emission that last read the scratch
     // fork / join of the ranking passes' stream in the captured launch sequence
-    cudaEvent_t fork[CPVS_MAX_LEVELS] = {nullptr}, join = nullptr, start = nullptr, cleared = nullptr, tables = nullptr, leaf_join = nullptr;
+    cudaEvent_t fork[CPVS_MAX_LEVELS] = {nullptr}, join = nullptr, start = nullptr, tables = nullptr, leaf_join = nullptr;
     bool tables_tuned = false;
     // single-pass levels: the levels >= small_lo run in the single-block
     // kernels; look-back tickets and flags (zeroed by every build)
@@ -3234,7 +3242,7 @@ void plan_release(Ctx& ctx, BuildPlan* P) {
     P->exec = nullptr;
     for (cudaEvent_t& e : P->fork)
         if (e) cudaEventDestroy(e), e = nullptr;
-    for (cudaEvent_t* e : {&P->join, &P->start, &P->cleared, &P->tables, &P->leaf_join})
+    for (cudaEvent_t* e : {&P->join, &P->start, &P->tables, &P->leaf_join})
         if (*e) cudaEventDestroy(*e), *e = nullptr;
     if (P->arena) ctx.release(P->arena, P->arena_bytes, true, nullptr);
     if (P->colrec) ctx.release(P->colrec, P->colrec_cap * 2 * sizeof(uint4), true, nullptr);
@@ -3489,6 +3497,7 @@ LeafColumns plan_leaf_columns(const BuildPlan* P) {
     lc.heavy_ctr = P->lmeta + 6;
     lc.any_nan = P->lmeta + 8;
     lc.kept = P->lkept;
+    lc.err = P->lmeta + 9;
     return lc;
 }
 
@@ -3540,9 +3549,32 @@ cpvs_status plan_enqueue(BuildPlan* P, cudaStream_t st, cudaStream_t rank_st, cu
         }
         CPVS_CUDA(clear(cr, rank_st));
     }
+    // the leaf classes of every column, beside the expansion (they need
+    // only the maps, their level-3 bounds and the cleared tables)
+    if (P->leafmasks) {
+        KernelTimer kt(tm, K_LEAF_COLUMNS, rank_st);
+        // one block per chunk of columns (the column records are sized to
+        // the batch's columns; a larger batch re-captures the sequence)
+        const uint32_t cg = (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>((P->colrec_cap + kColChunk - 1) / kColChunk, 8ull * P->max_grid));
+        CPVS_CUDA(launch_kernel(P->pow2 ? k_leaf_columns<true> : k_leaf_columns<false>, cg, kThreads, 0, rank_st, ch, 0,
+                                lc));
+    }
+    if (P->leafmasks) {
+        KernelTimer kt(tm, K_LEAF_COLUMNS, rank_st);
+        const uint32_t hg = (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>(P->colrec_cap / 64 + 1, P->max_grid));
+        CPVS_CUDA(launch_kernel(P->pow2 ? k_leaf_columns_heavy<true> : k_leaf_columns_heavy<false>, hg, kThreads, 0,
+                                rank_st, ch, 0, lc));
+    }
+    if (P->leafmasks) {
+        // the classes of the non-uniform runs (one thread each)
+        KernelTimer kt(tm, K_LEAF_CLASSES, rank_st);
+        CPVS_CUDA(launch_kernel(k_leaf_classes, plan_grid(P, P->cap[2], kThreads), kThreads, 0, rank_st, ch, 0, lc));
+    }
+    if (forked) CPVS_CUDA(cudaEventRecord(P->tables, rank_st));
     // results, level counts, job bases, look-back tickets and flags (the
-    // last two adjacent in the arena): before the first pass of either branch
-    // that may report an error there
+    // last two adjacent in the arena)
     {
         KernelTimer kt(tm, K_TABLE_CLEAR, st);
         ClearRanges cr{};
@@ -3556,36 +3588,6 @@ cpvs_status plan_enqueue(BuildPlan* P, cudaStream_t st, cudaStream_t rank_st, cu
         cr.n[3] = reinterpret_cast<const char*>(P->flags + P->flags_count) - reinterpret_cast<const char*>(P->tickets);
         CPVS_CUDA(clear(cr, st));
     }
-    if (forked) {
-        CPVS_CUDA(event(P->cleared));
-        CPVS_CUDA(cudaEventRecord(P->cleared, st));
-        CPVS_CUDA(cudaStreamWaitEvent(rank_st, P->cleared, 0));
-    }
-    // the leaf classes of every column, beside the expansion (they need
-    // only the maps, their level-3 bounds and the cleared tables)
-    if (P->leafmasks) {
-        KernelTimer kt(tm, K_LEAF_COLUMNS, rank_st);
-        // one block per chunk of columns (the column records are sized to
-        // the batch's columns; a larger batch re-captures the sequence)
-        const uint32_t cg = (uint32_t)std::max<uint64_t>(
-            1, std::min<uint64_t>((P->colrec_cap + kColChunk - 1) / kColChunk, 8ull * P->max_grid));
-        CPVS_CUDA(launch_kernel(P->pow2 ? k_leaf_columns<true> : k_leaf_columns<false>, cg, kThreads, 0, rank_st, ch, 0,
-                                lc, err));
-    }
-    if (P->leafmasks) {
-        KernelTimer kt(tm, K_LEAF_COLUMNS, rank_st);
-        const uint32_t hg = (uint32_t)std::max<uint64_t>(
-            1, std::min<uint64_t>(P->colrec_cap / 64 + 1, P->max_grid));
-        CPVS_CUDA(launch_kernel(P->pow2 ? k_leaf_columns_heavy<true> : k_leaf_columns_heavy<false>, hg, kThreads, 0,
-                                rank_st, ch, 0, lc));
-    }
-    if (P->leafmasks) {
-        // the classes of the non-uniform runs (one thread each)
-        KernelTimer kt(tm, K_LEAF_CLASSES, rank_st);
-        CPVS_CUDA(launch_kernel(k_leaf_classes, plan_grid(P, P->cap[2], kThreads), kThreads, 0, rank_st, ch, 0, lc,
-                                err));
-    }
-    if (forked) CPVS_CUDA(cudaEventRecord(P->tables, rank_st));
     // top-down: the small top levels as one cluster (which also places the
     // roots), then one pass per level
     const int Ls = P->small_lo;
@@ -3726,6 +3728,7 @@ cpvs_status plan_enqueue(BuildPlan* P, cudaStream_t st, cudaStream_t rank_st, cu
         KernelTimer kt(tm, K_LAYOUT, st);
         CPVS_CUDA(launch_kernel(k_layout, 1, 1024, 0, st, ch, 0, P->seg, P->lay, P->root_dev, njobs, P->bottom,
                                 static_cast<const LevelDev*>(P->lvt), rv.root_mask,
+                                P->leafmasks ? static_cast<const uint32_t*>(lc.err) : nullptr, err,
                                 reinterpret_cast<const uint4*>(P->res), reinterpret_cast<uint4*>(P->hout),
                                 (uint32_t)(result_bytes(njobs) / 16), P->ready()));
     }
@@ -4424,7 +4427,8 @@ extern "C" CPVS_API cpvs_status cpvs_shadow_build_noalloc(const float* depth, ui
         }
         k_dedup_remap<<<gi, kThreads, 0, st>>>(lv[L], counts, L, table);
     }
-    k_layout<<<1, 1024, 0, st>>>(seg, lay, root_dev, 1, bottom, nullptr, nullptr, nullptr, nullptr, 0, nullptr);
+    k_layout<<<1, 1024, 0, st>>>(seg, lay, root_dev, 1, bottom, nullptr, nullptr, nullptr, err, nullptr, nullptr, 0,
+                                 nullptr);
     CPVS_CUDA(cudaGetLastError());
     uint64_t hoff[2] = {0, 0};
     uint32_t hlu[2 * CPVS_MAX_LEVELS] = {0};

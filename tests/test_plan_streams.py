@@ -1,7 +1,7 @@
 """The order of a build's work over streams.  What one build of a plan leaves
 for the next is ordered by the plan's event alone, so everything that it leaves
-comes before the event's last record.  Within a build, the word that errors are
-reported in is cleared before any branch may report one."""
+comes before the event's last record.  Within a build, a word that errors are
+reported in is cleared before anything may report there."""
 import os
 import re
 
@@ -26,10 +26,15 @@ def test_the_level_table_is_copied_before_the_plans_event():
     assert b.rindex("cudaMemcpyAsync(P->lvt") < b.rindex("cudaEventRecord(P->done")
 
 
-def test_the_error_word_is_cleared_before_the_leaf_branch():
+def test_the_leaf_branch_reports_in_a_word_of_its_own():
+    """The results' region is cleared on the level chain's stream, beside the
+    branch: what the branch reports lies in what its own stream cleared before,
+    and the last kernel joins the two."""
     b = body("plan_enqueue")
-    clear, leaves = b.index("= P->res;"), b.index("k_leaf_columns<true>")
-    assert clear < b.index("cudaStreamWaitEvent(rank_st, P->cleared") < leaves
+    for launch in re.findall(r"launch_kernel\([^;]*k_leaf_(?:columns|classes)[^;]*;", b):
+        assert not re.search(r"\berr\b", launch), launch
+    assert b.index("P->lmeta + 4") < b.index("k_leaf_columns<true>")
+    assert "lc.err" in b[b.index("k_layout"):]
 
 
 @pytest.mark.gpu
