@@ -81,7 +81,7 @@ constexpr uint64_t kIndexKeep = 1ull << 30;  // 16 of the largest
 
 int* Ctx::lookup_choice(uint32_t num_levels, int depth, bool leafmasks, bool ndc, bool host_in, uint64_t n) {
     if (n < std::max(num_sms, 1) * 2048ull) return nullptr;  // 2048 threads to an SM
-    return &lookup_qpt_tuned[num_levels % CPVS_MAX_LEVELS][std::min(depth, kTopIndexDepth)][leafmasks][ndc][host_in];
+    return &lookup_qpt_tuned[(num_levels - (uint32_t)depth) % CPVS_MAX_LEVELS][leafmasks][ndc][host_in];
 }
 
 bool capturing(cudaStream_t st) {

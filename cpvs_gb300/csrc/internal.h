@@ -288,11 +288,14 @@ struct Ctx {
     // lookup queries per thread: fixed by cpvs_ctx_set_option, else tuned
     // once per kind of lookup
     int lookup_qpt = 0;
-    int lookup_qpt_tuned[CPVS_MAX_LEVELS][kTopIndexDepth + 1][2][2][2] = {};
+    int lookup_qpt_tuned[CPVS_MAX_LEVELS][2][2][2] = {};
     // Where the tuned number of such lookups is kept (0: not tuned yet); null:
-    // one query a thread, without timing.  The levels that the index leaves to
-    // the descent set the work, and the index's depth varies with a DAG's first
-    // batch.  Points read in place from host memory cross the host link with its
+    // one query a thread, without timing.  Kept by the levels that the index
+    // leaves to the descent: they set the work, and the index's depth varies with
+    // a DAG's first batch (2^24 points, a 1024^2 map: one query a thread is best
+    // with 6 levels in the index, 114.6 us against 121.1, two with all 7, 69.8
+    // against 72.6).  By side and depth both, maps of five sides had three times
+    // as many timings to sit through.  Points read in place from host memory cross the host link with its
     // latency, which favours more queries in flight per thread than points in
     // device memory do.  Batches whose queries are all in flight at once with
     // one a thread have nothing to gain from more, and take less than a timing's

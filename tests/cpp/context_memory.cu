@@ -147,15 +147,17 @@ static void pool_when_needed() {
 static void lookup_choice() {
     cpvs::Ctx c;
     c.num_sms = 152;
-    std::map<int*, int> places;
-    for (uint32_t levels = 2; levels <= 17; ++levels)
-        for (int depth = 0; depth <= 8; ++depth)
+    std::map<int*, std::vector<int>> places;
+    for (int levels = 2; levels <= 17; ++levels)
+        for (int depth = 0; depth <= 8 && depth < levels; ++depth)
             for (int k = 0; k < 8; ++k) {
                 check(!c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 500), "a small batch is not timed");
                 check(!c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 1 << 18), "a small batch is not timed");
-                ++places[c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 1 << 20)];
+                places[c.lookup_choice(levels, depth, k & 1, k & 2, k & 4, 1 << 20)].push_back(8 * (levels - depth) + k);
             }
-    check(places.size() == 16 * 9 * 8 && !places.count(nullptr), "a place for every kind");
+    check(places.size() == 17 * 8 && !places.count(nullptr), "a place for every kind");
+    for (const auto& p : places)
+        for (int kind : p.second) check(kind == p.second[0], "one kind to a place");
 }
 
 int main(int argc, char** argv) {
