@@ -861,24 +861,25 @@ cpvs_status cpvs_lookup_ndc_multi(const cpvs_shadow* const* shadows, uint32_t nu
     cudaStream_t st = (cudaStream_t)stream;
     cpvs_status r = set_device(ctx);
     if (r != CPVS_OK) return r;
-    // (a cell per point here: a descent beside others of other depths costs
-    // more; 2^22 points over 16 DAGs 63 -> 56 us, the first call 128 -> 132)
-    ensure_tops(shadows, num_shadows, st, kTopFactor, 2 * (n / num_shadows));
-    std::vector<cpvs::MultiDag> table(num_shadows);
-    for (uint32_t i = 0; i < num_shadows; ++i) table[i] = cpvs::shadow_table_entry(shadows[i]);
     cpvs::Ctx& c = ctx->c;
+    std::vector<cpvs::MultiDag> table(num_shadows);
     cpvs::MultiDag* dtab = nullptr;
     const uint64_t tb = num_shadows * sizeof(cpvs::MultiDag);
     if (!cpvs::multi_table_fits(num_shadows)) {
         r = c.alloc((void**)&dtab, tb, false, st);
         if (r != CPVS_OK) return r;
-        CPVS_CUDA(cudaMemcpyAsync(dtab, table.data(), tb, cudaMemcpyHostToDevice, st));
     }
     void* ids = nullptr;
     bool ids_own = false;
     r = stage_in(c, dag_index, n * 4, flags, st, &ids, &ids_own);
     if (r == CPVS_OK)
-        r = lookup_common(ctx, xyz, n, bits_out, flags, st, [&](const void* q, uint32_t* bits) {
+        r = lookup_common(ctx, xyz, n, bits_out, flags, st, [&](const void* q, uint32_t* bits) -> cpvs_status {
+            // (a cell per point here: a descent beside others of other depths
+            // costs more; 2^22 points over 16 DAGs 63 -> 56 us, the first call
+            // 128 -> 132)
+            ensure_tops(shadows, num_shadows, st, kTopFactor, 2 * (n / num_shadows));
+            for (uint32_t i = 0; i < num_shadows; ++i) table[i] = cpvs::shadow_table_entry(shadows[i]);
+            if (dtab) CPVS_CUDA(cudaMemcpyAsync(dtab, table.data(), tb, cudaMemcpyHostToDevice, st));
             return cpvs::launch_multi_lookup(table.data(), dtab, num_shadows, static_cast<const uint32_t*>(ids),
                                              static_cast<const float*>(q), n, bits, st, &c.timing);
         });
