@@ -879,7 +879,8 @@ cpvs_status cpvs_lookup_ndc_multi(const cpvs_shadow* const* shadows, uint32_t nu
             // 128 -> 132)
             ensure_tops(shadows, num_shadows, st, kTopFactor, 2 * (n / num_shadows));
             for (uint32_t i = 0; i < num_shadows; ++i) table[i] = cpvs::shadow_table_entry(shadows[i]);
-            if (dtab) CPVS_CUDA(cudaMemcpyAsync(dtab, table.data(), tb, cudaMemcpyHostToDevice, st));
+            const cpvs_status put = dtab ? cpvs::put_multi_table(table.data(), dtab, num_shadows, st) : CPVS_OK;
+            if (put != CPVS_OK) return put;
             return cpvs::launch_multi_lookup(table.data(), dtab, num_shadows, static_cast<const uint32_t*>(ids),
                                              static_cast<const float*>(q), n, bits, st, &c.timing);
         });

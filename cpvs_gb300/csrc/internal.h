@@ -160,6 +160,8 @@ struct MultiDag {
 // `host`: the table; `dags`: its device copy, needed (and read) only when
 // multi_table_fits is false.
 bool multi_table_fits(uint32_t ndags);
+// `host` into `dags`, in the order of `st`; `host` may go on return.
+cpvs_status put_multi_table(const MultiDag* host, MultiDag* dags, uint32_t ndags, cudaStream_t st);
 cpvs_status launch_multi_lookup(const MultiDag* host, const MultiDag* dags, uint32_t ndags, const uint32_t* ids,
                                 const float* xyz, uint64_t n, uint32_t* bits, cudaStream_t st,
                                 Timing* timing = nullptr);

@@ -843,6 +843,11 @@ struct MultiTable {
     MultiDag d[kMultiHeld];
 };
 
+// Entries of a table into memory from a launch's parameters.
+__global__ void k_put_table(const __grid_constant__ MultiTable tab, MultiDag* __restrict__ out, uint32_t count) {
+    if (threadIdx.x < count) out[threadIdx.x] = tab.d[threadIdx.x];
+}
+
 template <bool PARAM>
 __global__ void __launch_bounds__(kThreads)
     k_multi_lookup(const __grid_constant__ MultiTable tab, const MultiDag* __restrict__ dags, uint32_t ndags,
@@ -1070,6 +1075,22 @@ int tune_lookup(const uint32_t* dag, uint64_t words, uint32_t num_levels, bool l
 }
 
 bool multi_table_fits(uint32_t ndags) { return ndags <= kMultiHeld; }
+
+cpvs_status put_multi_table(const MultiDag* host, MultiDag* dags, uint32_t ndags, cudaStream_t st) {
+    // a recorded copy would read the caller's table when the graph runs
+    if (!capturing(st)) {
+        CPVS_CUDA(cudaMemcpyAsync(dags, host, ndags * sizeof(MultiDag), cudaMemcpyHostToDevice, st));
+        return CPVS_OK;
+    }
+    for (uint32_t at = 0; at < ndags; at += kMultiHeld) {
+        MultiTable tab{};
+        const uint32_t count = std::min(ndags - at, kMultiHeld);
+        std::copy(host + at, host + at + count, tab.d);
+        k_put_table<<<1, kMultiHeld, 0, st>>>(tab, dags + at, count);
+        CPVS_CUDA(cudaGetLastError());
+    }
+    return CPVS_OK;
+}
 
 cpvs_status launch_multi_lookup(const MultiDag* host, const MultiDag* dags, uint32_t ndags, const uint32_t* ids,
                                 const float* xyz, uint64_t n, uint32_t* bits, cudaStream_t st, Timing* timing) {

@@ -22,6 +22,45 @@ def test_no_index_is_made_in_a_capture():
         assert all(first < body.index(c) for c in ("alloc(", "tune_lookup(") if c in body), name
 
 
+def test_no_recorded_copy_of_a_calls_own_table():
+    with open(os.path.join(CSRC, "capi.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    body = text[re.search(r"cpvs_status cpvs_lookup_ndc_multi\([^;{]*\{", text).start():]
+    assert "cudaMemcpyAsync" not in body[:body.index("\n}\n")]
+    with open(os.path.join(CSRC, "lookup.cu")) as f:
+        text = f.read()
+    body = text[re.search(r"cpvs_status put_multi_table\([^;{]*\{", text).start():]
+    assert body.index("if (!capturing(st))") < body.index("cudaMemcpyAsync")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [64, 65, 150])
+def test_many_dags_in_a_graph(cp, count):
+    """A table larger than a launch's parameters: it is the graph's, whatever
+    becomes of the memory that the recording call had it in."""
+    import torch
+    ctx = cp.Context(0)
+    maps = [scene.rasterise(scene.make_scene(64, 0.9, 3 + k % 7, 1, seed=k)) for k in range(10)]
+    hs = cp.MinMaxHierarchy.create_batch(maps, ctx=ctx)
+    shadows = cp.CompressedShadow.create_batch(hs, [(k % 10, 0, 1) for k in range(count)])
+    g = torch.Generator("cuda").manual_seed(3)
+    pts = torch.rand((1 << 15, 3), device="cuda", generator=g) * 2 - 1
+    ids = torch.randint(count, (1 << 15,), device="cuda", generator=g, dtype=torch.int32)
+    want = cp.lookup_ndc_multi(shadows, ids, pts)
+    out = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        cp.lookup_ndc_multi(shadows, ids, pts, out=out, stream=stream)
+    junk = [np.full(count * 10, 0x5A5A5A5A, np.uint32) for _ in range(64)]
+    for _ in range(2):
+        out.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    del junk
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["ndc", "multi", "grid", "evaluate"])
 def test_first_lookup_in_a_graph(cp, oracle, kind):
