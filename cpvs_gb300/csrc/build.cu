@@ -1899,7 +1899,9 @@ __device__ __forceinline__ void load_child_ids(const LevelDev& child, uint32_t f
 // Signature hash of an inner node: job, child mask and the k child
 // identities in order.  A multilinear sum (one 32 x 32 -> 64 bit multiply-add
 // per term, independent of one another) through one 64-bit finaliser; equal
-// hashes are always compared, so its quality only sets the probe lengths.
+// hashes are always compared, so its quality only sets the probe lengths.  Any odd
+// multipliers do: among these are xxHash's 32-bit primes (K[0..2]) and halves of
+// wyhash's constants (the job's and the mask's), as published.
 __device__ __forceinline__ uint64_t inner_hash(uint32_t j, uint32_t m, uint32_t k, const uint32_t u[8]) {
     constexpr uint32_t K[8] = {0x9E3779B1u, 0x85EBCA77u, 0xC2B2AE3Du, 0xA54FF53Bu,
                                0xD1B54A33u, 0x8CB92BA7u, 0xF1357AEBu, 0xB5297A4Du};  // odd, above 2^31

@@ -11,7 +11,13 @@
  *   - All sizes are in elements unless named *_bytes.
  *   - `stream` is a cudaStream_t passed as void* (NULL = the legacy default
  *     stream).  Calls are stream-ordered; calls that return host data
- *     synchronise that stream before returning.
+ *     synchronise that stream before returning.  An object is used on other
+ *     streams than its own once the caller has ordered them behind its
+ *     creation; what a lookup adds to it (an index, on the first one) the
+ *     library orders itself.
+ *   - Lookups, grid evaluation and cpvs_shade with device buffers may be
+ *     recorded in a graph.  The first lookup outside a graph makes the index;
+ *     lookups recorded before it do without.
  *   - Pointers are host memory unless the call's flags say CPVS_IO_DEVICE
  *     (cpvs_shade, which has no flags, takes any buffer the GPU can reach).
  *     A plain pointer carries no size: each buffer must hold the elements
@@ -93,8 +99,10 @@ CPVS_API cpvs_status cpvs_ctx_set_budget(cpvs_ctx* ctx, uint64_t bytes);
 CPVS_API uint64_t cpvs_ctx_bytes_in_use(const cpvs_ctx* ctx);
 /* Tunable launch shapes; 0 (the default) = timed by the library.
  * CPVS_OPT_LOOKUP_QUERIES_PER_THREAD: independent descents each lookup
- * thread carries (1, 2 or 4); tuned per DAG depth by timing the three on the
- * first lookup batch of that depth.
+ * thread carries (1, 2 or 4); 1 for batches that it has all in flight at
+ * once, else tuned by timing the three on the first such batch (per levels
+ * that the DAG's lookup index leaves, NDC or voxel points, device or host
+ * memory).
  * CPVS_OPT_BUILD_CLUSTER_CAP: the largest level (planned nodes) that the
  * small-level cluster kernels take (2048, 4096, 8192 or 16384); larger
  * levels run in the multi-block kernels.
@@ -149,10 +157,9 @@ CPVS_API int cpvs_abi_version(void);
 CPVS_API cpvs_status cpvs_hierarchy_create(cpvs_ctx* ctx, const float* depth, uint32_t n, uint32_t flags, void* stream,
                                   cpvs_hierarchy** out);
 /* `count` hierarchies at once, map i of side sides[i] (sides may differ):
- * the same pyramids as cpvs_hierarchy_create per map, from one launch per
- * pyramid pass over every map's tiles (at most three per 256 maps) instead
- * of up to three per map -- the many-lights case, where the maps' own
- * launches dominate small maps.  flags: CPVS_IO_DEVICE (maps in device
+ * the same pyramids as cpvs_hierarchy_create per map, from one launch over
+ * every map's tiles (per 256 maps) instead of one per map -- the many-lights
+ * case, where the maps' own launches dominate small maps.  flags: CPVS_IO_DEVICE (maps in device
  * memory), CPVS_FLAG_BORROW_INPUT with it (read in place; the maps must
  * outlive the hierarchies).  On failure no hierarchy is returned. */
 CPVS_API cpvs_status cpvs_hierarchy_create_batch(cpvs_ctx* ctx, const float* const* depths, const uint32_t* sides,
@@ -262,7 +269,12 @@ CPVS_API cpvs_status cpvs_shadow_level_counts(const cpvs_shadow* s, uint64_t* tr
  * (src/CompressedShadow.h:64, src/CompressedShadow.cpp:404-463) and the
  * per-pixel descent of shader/traverse.cs:75-133; the NDC is quantised with
  * the reference's float32 order (src/CompressedShadowUtil.h:70-75).
- * `bits_out` holds ceil(n/32) words. */
+ * `bits_out` holds ceil(n/32) words.
+ * The DAG's first lookup lays out its index, which later ones use as it is: at
+ * most 8 times the DAG, or, without a budget, a cell per two points of that
+ * first batch (up to 64 MiB, and 1 GiB over all DAGs of the context).  A
+ * program that will look up 2^25 points and more does so first: 2^26 points
+ * take 0.39 ms then, 0.47 ms after a first batch of a few. */
 CPVS_API cpvs_status cpvs_shadow_lookup_ndc(const cpvs_shadow* s, const float* xyz, uint64_t n, uint32_t* bits_out,
                                    uint32_t flags, void* stream);
 /* Same, for integer voxel coordinates (the path getPathFromNDC yields),
