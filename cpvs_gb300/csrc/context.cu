@@ -91,6 +91,17 @@ bool capturing(cudaStream_t st) {
     return true;
 }
 
+bool reached(cudaEvent_t e) {
+    // another thread's capture is no reason to refuse the question, nor harmed
+    // by it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool done = cudaEventQuery(e) == cudaSuccess;
+    if (!done) cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return done;
+}
+
 cudaMemPool_t Ctx::index_source(uint64_t bytes) {
     if (bytes < kIndexOwn || budget) return nullptr;
     if (!index_pool && create_pool(device, &index_pool, kIndexKeep) != cudaSuccess) {

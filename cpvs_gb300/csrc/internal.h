@@ -280,6 +280,8 @@ cudaError_t create_pool(int device, cudaMemPool_t* pool, uint64_t keep);
 // Whether `st` is recording a graph (or may be: a legacy stream beside one
 // that is).
 bool capturing(cudaStream_t st);
+// Whether the work before the event's last record is done (false if unknown).
+bool reached(cudaEvent_t e);
 
 struct Ctx {
     Timing timing;

@@ -62,11 +62,10 @@ struct DeviceObject {
             const DeviceObject& o = *objects[i];
             if (!o.index_ || st == o.index_stream_ || !o.index_->event) continue;
             if (cpvs::capturing(st)) return;
-            if (cudaEventQuery(o.index_->event) == cudaSuccess) {
+            if (cpvs::reached(o.index_->event)) {
                 o.drop(o.index_);
                 continue;
             }
-            cudaGetLastError();  // (not ready)
             cudaStreamWaitEvent(st, o.index_->event, 0);
         }
     }

@@ -77,6 +77,45 @@ def test_first_lookups_on_two_streams(cp, oracle, case, kind):
 
 
 @pytest.mark.gpu
+def test_a_second_streams_lookup_beside_another_threads_capture(cp, case):
+    """The question whether an index is done, while another thread records a
+    graph: the lookup answers and the recording goes on."""
+    import torch
+    d, q, pts, want = case
+    ctx = cp.Context(0)
+    ctx.set_option(ctx.OPT_LOOKUP_QUERIES_PER_THREAD, 1)
+    sh = cp.CompressedShadow.from_depth(d, ctx=ctx)
+    out = torch.zeros(len(q) // 32, dtype=torch.int32, device="cuda")
+    a, b, c = (torch.cuda.Stream() for _ in range(3))
+    x = torch.ones(64, device="cuda")
+    torch.cuda.synchronize()
+    sh.lookup_ndc(pts, out=out, stream=a)
+    a.synchronize()
+    recording, asked, graph = threading.Event(), threading.Event(), torch.cuda.CUDAGraph()
+
+    def record():
+        with torch.cuda.graph(graph, stream=c):
+            x.add_(1)
+            recording.set()
+            asked.wait(20)
+            x.add_(1)
+
+    t = threading.Thread(target=record)
+    t.start()
+    assert recording.wait(20)
+    try:
+        sh.lookup_ndc(pts, out=out, stream=b)
+    finally:
+        asked.set()
+        t.join()
+    torch.cuda.synchronize()
+    assert np.array_equal(bits(cp, out, len(q)), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 3.0
+
+
+@pytest.mark.gpu
 def test_first_lookups_of_several_threads(cp, case):
     import torch
     d, q, pts, want = case
