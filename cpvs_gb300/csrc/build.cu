@@ -2903,10 +2903,8 @@ __global__ void k_layout(SegDev seg, JobLayout lay, const uint32_t* __restrict__
                          const LevelDev* __restrict__ lvt, uint32_t* root_mask, const uint32_t* leaf_err, uint32_t* err,
                          const uint4* res, uint4* host, uint32_t bytes16, uint32_t* ready) {
     chain_enter();
-    if (leaf_err && threadIdx.x == 0) {
-        const uint32_t e = __ldcg(leaf_err);
-        if (e) atomicOr(err, e);
-    }
+    // (read by a thread that seldom has a job, and used at the end)
+    const uint32_t leaf_bits = leaf_err && threadIdx.x == blockDim.x - 1u ? __ldcg(leaf_err) : 0u;
     // single block: each thread sums its jobs, then a block scan over jobs in
     // rounds of blockDim
     __shared__ uint32_t sm[64];
@@ -2941,6 +2939,7 @@ __global__ void k_layout(SegDev seg, JobLayout lay, const uint32_t* __restrict__
         carry += tot.x;
     }
     if (threadIdx.x == 0) lay.job_off[njobs] = carry;
+    if (leaf_bits) atomicOr(err, leaf_bits);
     if (!host) return;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < bytes16; i += blockDim.x) host[i] = __ldcg(res + i);

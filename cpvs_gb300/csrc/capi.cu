@@ -189,7 +189,6 @@ cpvs_status build_into_shadows(cpvs_ctx* ctx, const std::vector<cpvs::SourceSpec
 constexpr uint32_t kTopFactor = 8;
 void make_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor,
                uint64_t points) {
-    std::lock_guard<std::mutex> lock(shadows[0]->ctx->c.index_mutex);
     std::vector<cpvs::TopGrid> grids;
     std::vector<cpvs_shadow*> owners;
     for (size_t i = 0; i < count; ++i) {
@@ -240,6 +239,7 @@ void make_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st,
 // Indices for the shadows (of one context), and `st` after their making.
 void ensure_tops(const cpvs_shadow* const* shadows, size_t count, cudaStream_t st, uint32_t max_factor = kTopFactor,
                  uint64_t points = 0) {
+    std::lock_guard<std::mutex> lock(shadows[0]->ctx->c.index_mutex);
     make_tops(shadows, count, st, max_factor, points);
     DeviceObject::await_indices(shadows, count, st);
 }
@@ -1106,7 +1106,6 @@ cpvs_status cpvs_grid_words(const cpvs_grid* g, uint32_t* dag_out, uint64_t dag_
 // The grid's top index, built on its first lookup (stream-ordered).
 static void make_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     cpvs_grid* g = const_cast<cpvs_grid*>(cg);
-    std::lock_guard<std::mutex> lock(g->ctx->c.index_mutex);
     if (g->gtop || g->gtop_bytes == ~0ull || cpvs::capturing(st)) return;  // (as a shadow's)
     const int depth = cpvs::grid_top_depth(g->length, g->dag_levels, g->leafmasks, g->words);
     const uint64_t bytes = uint64_t(4) << (3 * (cpvs::log2_u32(g->length) + depth));
@@ -1125,6 +1124,7 @@ static void make_grid_top(const cpvs_grid* cg, cudaStream_t st) {
     DeviceObject::indexed_all(&g, 1, st);
 }
 static void ensure_grid_top(const cpvs_grid* g, cudaStream_t st) {
+    std::lock_guard<std::mutex> lock(g->ctx->c.index_mutex);
     make_grid_top(g, st);
     DeviceObject::await_indices(&g, 1, st);
 }

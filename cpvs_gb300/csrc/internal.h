@@ -348,8 +348,8 @@ struct Ctx {
     // budget) that there are, and the most of them.
     static constexpr uint64_t kIndexBeyond = 1ull << 30;
     uint64_t index_beyond = 0;
-    // Held while an object's index is made: lookups of several host threads may
-    // both be its first.
+    // Held while an object's index is made or awaited: lookups of several host
+    // threads may both be its first.
     std::mutex index_mutex;
     // The limit, 0 for none.  Under a limit the second pool holds no freed blocks.
     void set_budget(uint64_t bytes);

@@ -51,17 +51,16 @@ struct DeviceObject {
     static void indexed_all(T* const* objects, size_t count, cudaStream_t st) {
         record_all(objects, count, st, true);
     }
-    // Before a use of the indices of `objects` (of one context) on `st`.  (A
-    // capturing stream takes no wait for work outside its capture: what it
-    // records runs later.)
+    // Before a use of the indices of `objects` (of one context) on `st`, the
+    // context's index mutex held.  (A capturing stream takes no wait for work
+    // outside its capture: what it records runs later.)
     template <class T>
     static void await_indices(T* const* objects, size_t count, cudaStream_t st) {
-        if (!count) return;
-        std::lock_guard<std::mutex> lock(objects[0]->c_->event_mutex);
         for (size_t i = 0; i < count; ++i) {
             const DeviceObject& o = *objects[i];
             if (!o.index_ || st == o.index_stream_ || !o.index_->event) continue;
             if (cpvs::capturing(st)) return;
+            std::lock_guard<std::mutex> lock(o.c_->event_mutex);
             if (cpvs::reached(o.index_->event)) {
                 o.drop(o.index_);
                 continue;

@@ -17,11 +17,11 @@ def test_every_use_of_an_index_waits_for_it():
         text = re.sub(r"//[^\n]*", "", f.read())
     for name in ("ensure_tops", "ensure_grid_top"):
         body = text[re.search(r"void %s\([^;{]*\{" % name, text).start():]
-        assert "await_indices(" in body[:body.index("\n}\n")], name
+        body = body[:body.index("\n}\n")]
+        assert body.index("index_mutex") < body.index("make_") < body.index("await_indices("), name
     for name in ("make_tops", "make_grid_top"):
         body = text[re.search(r"void %s\([^;{]*\{" % name, text).start():]
-        body = body[:body.index("\n}\n")]
-        assert "index_mutex" in body and "indexed_all(" in body, name
+        assert "indexed_all(" in body[:body.index("\n}\n")], name
 
 
 @pytest.fixture(scope="module")
